@@ -46,38 +46,22 @@ namespace {
 // the batch kernel's rows per CTA
 int batch_rows(const mrlbm_batch* b) { return b->rows; }
 
-// shared memory and persistent grid of the batch kernel of each tile height
-template <int Q, typename T, int S, int TYI>
-mrlbm_status set_shape(mrlbm_batch* b, int sms)
-{
-    const int k = tile_kind(TYI);
-    b->smem[k] = ZSmem<Q, T, TYI, batch_npm<T, S>(), false, BATCH_STATIC_SMEM, batch_stages(Q)>::bytes;
-    cudaError_t e =
-        cudaFuncSetAttribute(batch_step<Q, T, S, TYI>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)b->smem[k]);
-    if (e != cudaSuccess) return fail(MRLBM_ECUDA, "batch attribute: %s", cudaGetErrorString(e));
-    int per_sm = 1;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, batch_step<Q, T, S, TYI>, 32 * (TYI + 2), b->smem[k]);
-    b->grid[k] = sms * std::max(per_sm, 1);
-    return MRLBM_OK;
-}
-
-template <int Q, typename T, int S = 0>
+// both tile heights' shared memory and persistent grid
 mrlbm_status set_shapes(mrlbm_batch* b, int sms)
 {
-    mrlbm_status st = set_shape<Q, T, S, TYI_BULK>(b, sms);
-    return st ? st : set_shape<Q, T, S, TYI_WALL>(b, sms);
+    if (b->lattice == 19)
+        return b->storage == MRLBM_F32    ? batch_shapes<19, float, 0>(b->smem, b->grid, sms)
+               : b->storage == MRLBM_F16U ? batch_shapes<19, __half, F_SPLITU>(b->smem, b->grid, sms)
+                                          : batch_shapes<19, __half, 0>(b->smem, b->grid, sms);
+    return b->storage == MRLBM_F32    ? batch_shapes<27, float, 0>(b->smem, b->grid, sms)
+           : b->storage == MRLBM_F16U ? batch_shapes<27, __half, F_SPLITU>(b->smem, b->grid, sms)
+                                      : batch_shapes<27, __half, 0>(b->smem, b->grid, sms);
 }
 
 template <int Q, typename T, int S = 0>
 void launch(mrlbm_batch* b)
 {
-    const int k = tile_kind(b->rows);
-    if (b->rows == TYI_BULK)
-        batch_step<Q, T, S, TYI_BULK>
-            <<<b->grid[k], 32 * (TYI_BULK + 2), b->smem[k], b->stream>>>(b->d_doms, b->d_items, b->d_ctl);
-    else
-        batch_step<Q, T, S, TYI_WALL>
-            <<<b->grid[k], 32 * (TYI_WALL + 2), b->smem[k], b->stream>>>(b->d_doms, b->d_items, b->d_ctl);
+    batch_launch<Q, T, S>(b->rows, b->smem, b->grid, b->d_doms, b->d_items, b->d_ctl, b->stream);
 }
 
 void launch_any(mrlbm_batch* b)
@@ -276,15 +260,7 @@ extern "C" mrlbm_status mrlbm_batch_create(int lattice, int storage, mrlbm_batch
     int dev = 0, sms = 148;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    mrlbm_status st;
-    if (lattice == 19)
-        st = storage == MRLBM_F32    ? set_shapes<19, float>(b, sms)
-             : storage == MRLBM_F16U ? set_shapes<19, __half, F_SPLITU>(b, sms)
-                                     : set_shapes<19, __half>(b, sms);
-    else
-        st = storage == MRLBM_F32    ? set_shapes<27, float>(b, sms)
-             : storage == MRLBM_F16U ? set_shapes<27, __half, F_SPLITU>(b, sms)
-                                     : set_shapes<27, __half>(b, sms);
+    const mrlbm_status st = set_shapes(b, sms);
     if (st) { delete b; return st; }
     if (cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking) != cudaSuccess ||
         cudaEventCreate(&b->ev0) != cudaSuccess || cudaEventCreate(&b->ev1) != cudaSuccess ||

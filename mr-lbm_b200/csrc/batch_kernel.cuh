@@ -6,6 +6,7 @@
 // last CTA to finish resets the counter and advances the batch step, so the
 // launch can be replayed from a CUDA graph with no host work between steps.
 #pragma once
+#include "../../include/mrlbm.h"
 #include "kernels.cuh"
 
 namespace mrlbm {
@@ -60,6 +61,8 @@ __device__ __forceinline__ bool batch_column(
     const ZSmem<Q, T, TYI, batch_npm<T, FLAGS & F_SPLITU>(), false, BATCH_STATIC_SMEM, batch_stages(Q)>& sm,
     unsigned& g0)
 {
+    if constexpr (sums_march(Q, FLAGS))
+        return sum_column<T, FLAGS, TYI, 1>(a, map, it.X0, it.Y0, it.z0, min(it.z0 + a.lz, a.nz), sm, g0);
     // one generic-pointer solve for every flag set: the batch kernel holds
     // them all, and two inlined solves per set spill
     using BCP = std::conditional_t<batch_stages(Q), TableBCGeneric, TableBC>;
@@ -135,5 +138,12 @@ __global__ void __launch_bounds__(32 * (TYI + 2), ctas_per_sm(TYI))
         }
     }
 }
+
+// shape and launch (batch_dispatch.cuh), instantiated per lattice and storage
+template <int Q, typename T, int S>
+mrlbm_status batch_shapes(size_t* smem, int* grid, int sms);
+template <int Q, typename T, int S>
+void batch_launch(int rows, const size_t* smem, const int* grid, const BatchDomain* doms, const BatchItem* items,
+                  BatchCtl* ctl, cudaStream_t s);
 
 }  // namespace mrlbm

@@ -377,7 +377,10 @@ extern "C" mrlbm_status mrlbm_save_info(mrlbm_domain* dom, const char* path_file
     StepArgs sa;
     int flags = 0;
     fill_step_args(dom, sa, dom->cur, flags);
-    const std::string t = info_text(dom->d, id_sim, case_name, nsteps, mlups, tile_rows(flags), sa.lz);
+    // the nominal tile of the flag set (the sums march has a z chunk of its own), as in mrlbm_info_text
+    const int kind = tile_kind(tile_rows(flags));
+    const int lz = dom->lz > 0 ? dom->lz : tile_ordered(dom, flags) ? dom->lz_o[kind] : dom->lz_t[kind];
+    const std::string t = info_text(dom->d, id_sim, case_name, nsteps, mlups, tile_rows(flags), lz);
     return write_file(std::string(path_files) + "/" + id_sim + "/" + id_sim + "_info.txt", t.data(), t.size());
 }
 

@@ -96,9 +96,10 @@ __host__ __device__ constexpr int ctas_per_sm(int tyi) { return tyi <= 8 ? 2 : 1
 // dynamic shared memory a CTA may take: the opt-in per-block limit for one
 // CTA per SM, else an even share of the SM's 228 KB less the 1 KB each
 // block reserves
+__host__ __device__ constexpr size_t smem_share(int ctas) { return ctas == 1 ? 232448 : 233472 / ctas / 128 * 128 - 1024; }
 __host__ __device__ constexpr size_t smem_budget(int tyi)
 {
-    return ctas_per_sm(tyi) == 1 ? 232448 : 233472 / ctas_per_sm(tyi) - 1024;
+    return smem_share(ctas_per_sm(tyi));
 }
 // stored moments and moment pairs of a flag set
 __host__ __device__ constexpr int nmoments_of(int flags)
@@ -107,6 +108,11 @@ __host__ __device__ constexpr int nmoments_of(int flags)
            ((flags & F_SPLITU) ? ((flags & (F_POWERLAW | F_BINGHAM)) ? 4 : 3) : 0);
 }
 __host__ __device__ constexpr int npairs_of(int flags) { return (nmoments_of(flags) + 1) / 2; }
+// flag sets of the sums march (sum_march.cuh)
+__host__ __device__ constexpr bool sums_march(int q, int flags)
+{
+    return q == 27 && (flags & ~(F_FORCE | F_SPLITU)) == 0;
+}
 // index of a tile height among the domain's tensor maps and z chunks
 __host__ __device__ constexpr int tile_kind(int tyi) { return tyi == TYI_BULK ? 0 : 1; }
 __host__ __device__ constexpr int tile_rows_of_kind(int kind) { return kind == 0 ? TYI_BULK : TYI_WALL; }
@@ -250,6 +256,10 @@ constexpr bool scaled_storage()
 {
     return std::is_same<T, __half>::value;
 }
+
+constexpr float F16_SCALE_RHO = 256.0f, F16_SCALE_U = 8.0f, F16_SCALE_PI = 64.0f;
+// split storage: a low word's scale over its high word's
+constexpr float F16_SCALE_LOW = 2048.0f;
 
 // a moment pair of one node: 8 bytes (FP32) or 4 bytes (FP16 / BF16)
 template <typename T>
@@ -1141,6 +1151,67 @@ __device__ __forceinline__ void store_node(const StepArgs& a, long long idx, con
     for (int m = 0; m < NM; m++) Stor<T>::st(outp + mphys(m, idx, a.field), o[m]);
 }
 
+// The ghost copies of a finished node on a face of a periodic axis (gx, gy,
+// gz: on a face of that axis): the shell stays equal to the wrapped interior.
+template <typename T, int NM>
+__device__ __forceinline__ void store_ghosts(const StepArgs& a, bool gx, bool gy, bool gz, int x, int y, int zd,
+                                             const float* o)
+{
+    if ((gx && a.nx == 1) || (gy && a.ny == 1) || (gz && a.nz == 1)) {
+        // degenerate one-node axis: the node has both ghost copies
+#pragma unroll 1
+        for (int iz = 0; iz < 3; iz++)
+#pragma unroll 1
+            for (int iy = 0; iy < 3; iy++)
+#pragma unroll 1
+                for (int ix = 0; ix < 3; ix++) {
+                    const bool vz = iz == 0 || (gz && (iz == 1 ? zd == 0 : zd == a.nz - 1));
+                    const bool vy = iy == 0 || (gy && (iy == 1 ? y == 0 : y == a.ny - 1));
+                    const bool vx = ix == 0 || (gx && (ix == 1 ? x == 0 : x == a.nx - 1));
+                    if (!(vx && vy && vz) || (ix == 0 && iy == 0 && iz == 0)) continue;
+                    const int cz = iz == 0 ? zd : (iz == 1 ? a.nz : -1);
+                    const int cy = iy == 0 ? y : (iy == 1 ? a.ny : -1);
+                    const int cxx = ix == 0 ? x : (ix == 1 ? a.nx : -1);
+                    store_node<T, NM>(a, pidx(cxx, cy, cz, a.pitch, a.plane), o);
+                }
+    } else {
+        const int xa = x == 0 ? a.nx : -1, ya = y == 0 ? a.ny : -1, za = zd == 0 ? a.nz : -1;
+        if (gx) store_node<T, NM>(a, pidx(xa, y, zd, a.pitch, a.plane), o);
+        if (gy) store_node<T, NM>(a, pidx(x, ya, zd, a.pitch, a.plane), o);
+        if (gz) store_node<T, NM>(a, pidx(x, y, za, a.pitch, a.plane), o);
+        if (gx && gy) store_node<T, NM>(a, pidx(xa, ya, zd, a.pitch, a.plane), o);
+        if (gx && gz) store_node<T, NM>(a, pidx(xa, y, za, a.pitch, a.plane), o);
+        if (gy && gz) store_node<T, NM>(a, pidx(x, ya, za, a.pitch, a.plane), o);
+        if (gx && gy && gz) store_node<T, NM>(a, pidx(xa, ya, za, a.pitch, a.plane), o);
+    }
+}
+
+// A finished node's words as stored (o: the collided moments in the stored
+// scaling): the split storage's low words and the storage scale.
+template <typename T, int NM, int FLAGS>
+__device__ __forceinline__ void stored_words(const StepArgs& a, float* o)
+{
+    if constexpr ((FLAGS & F_SPLITU) != 0) split_words<NM, nmoments_of(FLAGS & ~F_SPLITU)>(a, o);
+    if constexpr (scaled_storage<T>()) {
+#pragma unroll
+        for (int m = 0; m < NM; m++) o[m] = o[m] * a.scale[m];
+    }
+}
+
+// A finished node: its words, the store and its ghost copies.
+template <typename T, int NM, int FLAGS>
+__device__ __forceinline__ void finish_node(const StepArgs& a, bool live, int x, int y, int zd, unsigned oidx, float* o)
+{
+    stored_words<T, NM, FLAGS>(a, o);
+    if (live) {
+        store_node32<T, NM>(a, oidx, o);
+        const bool gx = (a.periodic & 1) && (x == 0 || x == a.nx - 1);
+        const bool gy = (a.periodic & 2) && (y == 0 || y == a.ny - 1);
+        const bool gz = (a.periodic & 4) && (zd == 0 || zd == a.nz - 1);
+        if (gx || gy || gz) store_ghosts<T, NM>(a, gx, gy, gz, x, y, zd, o);
+    }
+}
+
 // Consumption of plane k (second half): the c_y != 0 populations arriving from
 // the neighbouring rows are read from exchange buffer k&1; with gsh they
 // complete the populations that plane k sends.  Those with c_z = -1 complete
@@ -1250,47 +1321,7 @@ __device__ __forceinline__ void prod_b(const StepArgs& a, int k, int zp, const f
             o[10] = tC;
             o[11] = tq[0]; o[12] = tq[1]; o[13] = tq[2];
         }
-        if constexpr ((FLAGS & F_SPLITU) != 0) split_words<NM, nmoments_of(FLAGS & ~F_SPLITU)>(a, o);
-        if constexpr (scaled_storage<T>()) {
-#pragma unroll
-            for (int m = 0; m < NM; m++) o[m] = o[m] * a.scale[m];
-        }
-        if (live && cls != CLS_SOLID) {
-            store_node32<T, NM>(a, oidx, o);
-            // periodic axes: keep the ghost shell equal to the wrapped interior
-            const bool gx = (a.periodic & 1) && (x == 0 || x == a.nx - 1);
-            const bool gy = (a.periodic & 2) && (y == 0 || y == a.ny - 1);
-            const bool gz = (a.periodic & 4) && (zd == 0 || zd == a.nz - 1);
-            if (gx || gy || gz) {
-                if ((gx && a.nx == 1) || (gy && a.ny == 1) || (gz && a.nz == 1)) {
-                    // degenerate one-node axis: the node has both ghost copies
-#pragma unroll 1
-                    for (int iz = 0; iz < 3; iz++)
-#pragma unroll 1
-                        for (int iy = 0; iy < 3; iy++)
-#pragma unroll 1
-                            for (int ix = 0; ix < 3; ix++) {
-                                const bool vz = iz == 0 || (gz && (iz == 1 ? zd == 0 : zd == a.nz - 1));
-                                const bool vy = iy == 0 || (gy && (iy == 1 ? y == 0 : y == a.ny - 1));
-                                const bool vx = ix == 0 || (gx && (ix == 1 ? x == 0 : x == a.nx - 1));
-                                if (!(vx && vy && vz) || (ix == 0 && iy == 0 && iz == 0)) continue;
-                                const int cz = iz == 0 ? zd : (iz == 1 ? a.nz : -1);
-                                const int cy = iy == 0 ? y : (iy == 1 ? a.ny : -1);
-                                const int cxx = ix == 0 ? x : (ix == 1 ? a.nx : -1);
-                                store_node<T, NM>(a, pidx(cxx, cy, cz, a.pitch, a.plane), o);
-                            }
-                } else {
-                    const int xa = x == 0 ? a.nx : -1, ya = y == 0 ? a.ny : -1, za = zd == 0 ? a.nz : -1;
-                    if (gx) store_node<T, NM>(a, pidx(xa, y, zd, a.pitch, a.plane), o);
-                    if (gy) store_node<T, NM>(a, pidx(x, ya, zd, a.pitch, a.plane), o);
-                    if (gz) store_node<T, NM>(a, pidx(x, y, za, a.pitch, a.plane), o);
-                    if (gx && gy) store_node<T, NM>(a, pidx(xa, ya, zd, a.pitch, a.plane), o);
-                    if (gx && gz) store_node<T, NM>(a, pidx(xa, y, za, a.pitch, a.plane), o);
-                    if (gy && gz) store_node<T, NM>(a, pidx(x, ya, za, a.pitch, a.plane), o);
-                    if (gx && gy && gz) store_node<T, NM>(a, pidx(xa, ya, za, a.pitch, a.plane), o);
-                }
-            }
-        }
+        finish_node<T, NM, FLAGS>(a, live && cls != CLS_SOLID, x, y, zd, oidx, o);
     }
     // advance the z pipeline: the consumed U(zp-2) slot now holds U(zp)
     static_for<0, Q>([&](auto I) {
@@ -1354,6 +1385,8 @@ struct ZSmem {
     float* exg1;
     float4* edge;   // flow edge buffer
     float4* edgeg;  // thermal edge buffer (TH only)
+    // edge buffer of a sums-march column (sum_march.cuh): it has no row exchange
+    __device__ __forceinline__ float* sum_edge() const { return reinterpret_cast<float*>(ex4); }
     __device__ __forceinline__ explicit ZSmem(unsigned char* smem)
     {
         bars = reinterpret_cast<uint64_t*>(smem);
@@ -1369,30 +1402,20 @@ struct ZSmem {
 
 
 
-// Per-CTA pipeline state of the z-march over one column.  The TMA ring is
-// indexed by a running production count `g0 + k` so a persistent CTA can
-// chain columns without re-initialising its mbarriers.  Warps 0 .. TYI-1 run
-// the interior pipeline (interior_loop), warps TYI and TYI+1 the helper one
-// (helper_loop); both take the same barriers in the same order.
-template <int Q, typename T, int FLAGS, int TYI, typename BCP, int NPM, int RES = 0, bool WC = false>
-struct ZMarch {
+// The TMA ring of a column's planes.  It is indexed by a running production
+// count `g0 + k`, so a persistent CTA can chain columns without
+// re-initialising its mbarriers.  Lane 0 of warp PW (the first helper) issues
+// the loads.  NP: moment pairs in a stage row; SM: the shared-memory carve-up.
+template <typename T, int TYI, int NP, typename SM, int PW = TYI>
+struct ZRing {
     static constexpr int NR = TYI + 2;
     static constexpr int BX = box_x<T>();
-    static constexpr int NUP = lat_num_cz(Q, 1);
-    static constexpr int NMID = lat_num_cz(Q, 0);
-    static constexpr bool OMF = (FLAGS & (F_POWERLAW | F_BINGHAM)) != 0;
-    static constexpr bool TH = (FLAGS & F_THERMAL) != 0;
-    static constexpr int NM = nmoments_of(FLAGS);
-    static constexpr int NML = nmoments_of(FLAGS & ~F_SPLITU);  // moments before the split storage's low words
-    static constexpr int NP = (NM + 1) / 2;  // moment pairs in a stage row
     static constexpr int ROW = NP * 2 * BX;  // elements of a stage row
     static constexpr size_t stage_bytes = (size_t)NR * ROW * sizeof(T);
-    using EX = Exchange<Q, TYI>;
-    using EXG = Exchange<19, TYI>;
-    using SM = ZSmem<Q, T, TYI, NPM, TH, RES, WC>;
     static constexpr int NS = SM::NS;
-    static constexpr int TMA_THREAD = 32 * TYI;  // lane 0 of the bottom helper
-    static_assert(NP <= NPM, "ring slots sized for fewer moment pairs");
+    static constexpr size_t ring_stride = SM::stage_max;
+    static constexpr int TMA_THREAD = 32 * PW;  // lane 0 of the first helper
+    static_assert(stage_bytes <= SM::stage_max, "ring slots sized for fewer moment pairs");
 
     const StepArgs& a;
     const CUtensorMap* map;
@@ -1402,9 +1425,19 @@ struct ZMarch {
     int cs;           // ring slot of the next production to wait for
     unsigned cph;     // its mbarrier phase parity
 
+    __device__ __forceinline__ ZRing(const StepArgs& a_, const CUtensorMap* map_, const SM& sm_, unsigned g0_, int X0_,
+                                     int Y0_, int z0_, int zend)
+        : a(a_), map(map_), sm(sm_), g0(g0_), X0(X0_), Y0(Y0_), z0(z0_), nprod(zend - z0_ + 2 /* planes z0-1 .. zend */)
+    {
+        // aligned box start (padded column): the TMA x coordinate, 2 elements a
+        // node, must be a multiple of 16 bytes
+        constexpr int NODE_ALIGN = 8 / (int)sizeof(T);
+        p0 = (X0 - 1 + XOFF) & ~(NODE_ALIGN - 1);
+        cs = slot(0);
+        cph = phase(0);
+    }
     __device__ __forceinline__ int slot(int k) const { return (int)((g0 + (unsigned)k) % NS); }
     __device__ __forceinline__ unsigned phase(int k) const { return ((g0 + (unsigned)k) / NS) & 1u; }
-    static constexpr size_t ring_stride = SM::stage_max;
     __device__ __forceinline__ const T* stage_base() const { return reinterpret_cast<const T*>(sm.stages + cs * ring_stride); }
     // element offset of node x of stage row er (pair of moments 0, 1)
     __device__ __forceinline__ int stage_off(int er, int x) const { return er * ROW + 2 * ((x + XOFF) - p0); }
@@ -1414,7 +1447,15 @@ struct ZMarch {
         // x runs over the interleaved pair elements: 2 per node
         tma_load_4d(sm.stages + s * ring_stride, map, 2 * p0, 0, Y0, z0 + k, &sm.bars[s]);
     }
-    __device__ __forceinline__ void load(int k) const { load_slot(slot(k), k); }
+    // the column's first loads
+    __device__ __forceinline__ void fill() const
+    {
+        if (threadIdx.x == TMA_THREAD) {
+            // the ring was last read through the generic proxy (previous column)
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            for (int s = 0; s < NS && s < nprod; s++) load_slot(slot(s), s);
+        }
+    }
     // CTA-wide timeout flag next to the ring barriers: a thread whose bounded
     // wait gave up raises it before the per-plane barrier, every thread reads
     // it after (a plain barrier measured 3 % faster than a reducing one)
@@ -1433,6 +1474,48 @@ struct ZMarch {
             cph ^= 1u;
         }
     }
+    // a bounded wait gave up in production kfail: flag it and give the copies
+    // still in flight a bounded time to land
+    __device__ __forceinline__ void drain(int kfail) const
+    {
+        if (threadIdx.x == TMA_THREAD) {
+            atomicOr(a.err, 1);
+            for (int q = kfail; q < nprod && q < kfail + NS; q++) (void)mbar_wait(&sm.bars[slot(q)], phase(q));
+        }
+    }
+};
+
+// Per-CTA pipeline state of the z-march over one column.  Warps 0 .. TYI-1 run
+// the interior pipeline (interior_loop), warps TYI and TYI+1 the helper one
+// (helper_loop); both take the same barriers in the same order.
+template <int Q, typename T, int FLAGS, int TYI, typename BCP, int NPM, int RES = 0, bool WC = false>
+struct ZMarch : ZRing<T, TYI, npairs_of(FLAGS), ZSmem<Q, T, TYI, NPM, (FLAGS & F_THERMAL) != 0, RES, WC>> {
+    using SM = ZSmem<Q, T, TYI, NPM, (FLAGS & F_THERMAL) != 0, RES, WC>;
+    using Ring = ZRing<T, TYI, npairs_of(FLAGS), SM>;
+    using Ring::NR;
+    using Ring::a;
+    using Ring::sm;
+    using Ring::X0;
+    using Ring::Y0;
+    using Ring::z0;
+    using Ring::nprod;
+    using Ring::cs;
+    using Ring::cph;
+    using Ring::stage_base;
+    using Ring::stage_off;
+    using Ring::raise_timeout;
+    using Ring::timed_out;
+    using Ring::advance;
+    using Ring::Ring;
+    static constexpr int NUP = lat_num_cz(Q, 1);
+    static constexpr int NMID = lat_num_cz(Q, 0);
+    static constexpr bool OMF = (FLAGS & (F_POWERLAW | F_BINGHAM)) != 0;
+    static constexpr bool TH = (FLAGS & F_THERMAL) != 0;
+    static constexpr int NM = nmoments_of(FLAGS);
+    static constexpr int NML = nmoments_of(FLAGS & ~F_SPLITU);  // moments before the split storage's low words
+    using EX = Exchange<Q, TYI>;
+    using EXG = Exchange<19, TYI>;
+
     // end of pipeline step k: barrier, timeout check, ring advance
     __device__ __forceinline__ bool end_step(int k, bool ok)
     {
@@ -1630,13 +1713,7 @@ __device__ __forceinline__ bool zmarch_column(const StepArgs& a, const CUtensorM
 {
     using ZM = ZMarch<Q, T, FLAGS, TYI, BCP, NPM, RES, WC>;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    // aligned box start (padded column): the TMA x coordinate, 2 elements a
-    // node, must be a multiple of 16 bytes
-    constexpr int NODE_ALIGN = 8 / (int)sizeof(T);
-    const int p0 = (X0 - 1 + XOFF) & ~(NODE_ALIGN - 1);
-    ZM zm{a, map, sm, g0, X0, Y0, z0, p0, zend - z0 + 2 /* planes z0-1 .. zend */, 0, 0u};
-    zm.cs = zm.slot(0);
-    zm.cph = zm.phase(0);
+    ZM zm(a, map, sm, g0, X0, Y0, z0, zend);
 #ifdef MRLBM_BOUNDS_CHECK
     if (threadIdx.x == 0) {
         using SMT = ZSmem<Q, T, TYI, NPM, (FLAGS & F_THERMAL) != 0, RES, WC>;
@@ -1655,22 +1732,14 @@ __device__ __forceinline__ bool zmarch_column(const StepArgs& a, const CUtensorM
     __syncthreads();
 #endif
 
-    if (threadIdx.x == ZM::TMA_THREAD) {
-        // the ring was last read through the generic proxy (previous column)
-        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-        for (int s = 0; s < ZM::NS && s < zm.nprod; s++) zm.load(s);
-    }
+    zm.fill();
     int kfail;
     if (warp < TYI) kfail = zm.interior_loop(lane, warp);
     else if (warp == TYI) kfail = zm.template helper_loop<-1>(lane);
     else kfail = zm.template helper_loop<1>(lane);
     if (kfail >= 0) {
-        // a bounded wait gave up: flag it, give the copies still in flight a
-        // bounded time to land, and leave together
-        if (threadIdx.x == ZM::TMA_THREAD) {
-            atomicOr(a.err, 1);
-            for (int q = kfail; q < zm.nprod && q < kfail + ZM::NS; q++) (void)mbar_wait(&sm.bars[zm.slot(q)], zm.phase(q));
-        }
+        // a bounded wait gave up: leave together
+        zm.drain(kfail);
         __syncthreads();
         return false;
     }
@@ -1680,13 +1749,17 @@ __device__ __forceinline__ bool zmarch_column(const StepArgs& a, const CUtensorM
     return true;
 }
 
+}  // namespace mrlbm
+
+#include "sum_march.cuh"
+
+namespace mrlbm {
+
 // Barriers, the timeout flag and, in wall kernels, the staged copy of the
 // first ZSmem::CT classes of the table bc (nbc classes)
-template <int Q, typename T, int TYI, int NPM, bool TH, int RES, bool WC>
-__device__ __forceinline__ void zmarch_init_barriers(const ZSmem<Q, T, TYI, NPM, TH, RES, WC>& sm,
-                                                     const BcClass* bc = nullptr, int nbc = 0)
+template <typename SMT>
+__device__ __forceinline__ void zmarch_init_barriers(const SMT& sm, const BcClass* bc = nullptr, int nbc = 0)
 {
-    using SMT = ZSmem<Q, T, TYI, NPM, TH, RES, WC>;
     int staged = 0;
     if constexpr (SMT::CT > 0) {
         staged = nbc < SMT::CT ? nbc : SMT::CT;
@@ -1784,17 +1857,32 @@ __device__ __forceinline__ void tile_order_end(const StepArgs& a, int tx, int ty
     }
 }
 
+// Launch shape of the single-domain step: warps of a CTA and CTAs per SM
+__host__ __device__ constexpr int step_warps(int q, int flags, int tyi)
+{
+    return sums_march(q, flags) ? tyi / SUM_ROWS + 1 : tyi + 2;
+}
+__host__ __device__ constexpr int step_ctas(int q, int flags, int tyi)
+{
+    return sums_march(q, flags) ? SUM_CTAS : ctas_per_sm(tyi);
+}
+
+template <int Q, typename T, int FLAGS, int TYI, typename BCP>
+using step_smem_t =
+    std::conditional_t<sums_march(Q, FLAGS), SumSmem<T, TYI, npairs_of(FLAGS)>,
+                       ZSmem<Q, T, TYI, npairs_of(FLAGS), (FLAGS & F_THERMAL) != 0, 0,
+                             (FLAGS & F_BC) != 0 && stages_classes<BCP>::value>>;
+
 // Single-domain step: one CTA per (x tile, y tile, z chunk of lz planes).
 // Launch order runs x tiles fastest, so the CTAs resident at one time march
 // neighbouring columns through the same planes and their halo reads hit L2.
 // With a.sched set, a CTA's tile comes from its ticket instead (tile_order_begin).
 template <int Q, typename T, int FLAGS, int TYI, typename BCP = TableBC>
-__global__ void __launch_bounds__(32 * (TYI + 2), ctas_per_sm(TYI))
+__global__ void __launch_bounds__(32 * step_warps(Q, FLAGS, TYI), step_ctas(Q, FLAGS, TYI))
     zmarch_step(const __grid_constant__ CUtensorMap map_in, const StepArgs a)
 {
     extern __shared__ __align__(128) unsigned char smem[];
-    constexpr bool WC = (FLAGS & F_BC) != 0 && stages_classes<BCP>::value;
-    const ZSmem<Q, T, TYI, npairs_of(FLAGS), (FLAGS & F_THERMAL) != 0, 0, WC> sm(smem);
+    const step_smem_t<Q, T, FLAGS, TYI, BCP> sm(smem);
     int tx = blockIdx.x, ty = blockIdx.y, kc = blockIdx.z;
     unsigned s = 0;
     if (a.sched) s = tile_order_begin(a, tx, ty, kc);
@@ -1803,9 +1891,12 @@ __global__ void __launch_bounds__(32 * (TYI + 2), ctas_per_sm(TYI))
     // thread through the generic proxy; the ring's loads use the async one
     if (a.sched) asm volatile("fence.proxy.async.global;" ::: "memory");
     unsigned g0 = 0;
-    const int z0 = kc * a.lz;
-    (void)zmarch_column<Q, T, FLAGS, TYI, BCP>(a, &map_in, tx * TILE_X, ty * TYI, z0, min(z0 + a.lz, a.nz), sm, g0);
-    // zmarch_column ends with a CTA barrier on every path
+    const int z0 = kc * a.lz, zend = min(z0 + a.lz, a.nz);
+    if constexpr (sums_march(Q, FLAGS))
+        (void)sum_column<T, FLAGS, TYI, SUM_ROWS>(a, &map_in, tx * TILE_X, ty * TYI, z0, zend, sm, g0);
+    else
+        (void)zmarch_column<Q, T, FLAGS, TYI, BCP>(a, &map_in, tx * TILE_X, ty * TYI, z0, zend, sm, g0);
+    // the column ends with a CTA barrier on every path
     if (a.sched) tile_order_end(a, tx, ty, kc, s);
 }
 
@@ -1818,8 +1909,7 @@ __host__ __device__ inline dim3 zmarch_grid(int nx, int ny, int nz, int tyi, int
 template <int Q, typename T, int FLAGS, int TYI, typename BCP = TableBC>
 constexpr size_t step_smem_bytes()
 {
-    return ZSmem<Q, T, TYI, npairs_of(FLAGS), (FLAGS & F_THERMAL) != 0, 0,
-                 (FLAGS & F_BC) != 0 && stages_classes<BCP>::value>::bytes;
+    return step_smem_t<Q, T, FLAGS, TYI, BCP>::bytes;
 }
 
 }  // namespace mrlbm

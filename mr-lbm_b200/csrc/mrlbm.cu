@@ -1,6 +1,7 @@
 // mrlbm.cu -- C ABI (include/mrlbm.h) over the sm_100a MR-LBM kernels.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cmath>
 #include <cstdarg>
 #include <cstdio>
@@ -226,13 +227,13 @@ void mrlbm::storage_scales(int storage, int nm, float* scale, float* iscale)
             // powers of two keep values of the shifted moments in the normal
             // range of fp16 (exact, no rounding from the scaling itself);
             // bf16 has fp32's exponent range and needs none
-            s = k == 0 ? 256.0f : (k <= 3 ? 8.0f : (k <= 9 ? 64.0f : 1.0f));
+            s = k == 0 ? F16_SCALE_RHO : (k <= 3 ? F16_SCALE_U : (k <= 9 ? F16_SCALE_PI : 1.0f));
             // split storage: the low words of 3u and omega (stored after the
             // nm moments) are what the high word rounds away, at most half
             // an fp16 ulp of the scaled value, so 2^11 times the high word's
             // scale keeps them in fp16's normal range
-            if (storage == MRLBM_F16U && k >= nm && k < nm + 3) s = 8.0f * 2048.0f;
-            if (storage == MRLBM_F16U && nm == 11 && k == nm + 3) s = 2048.0f;
+            if (storage == MRLBM_F16U && k >= nm && k < nm + 3) s = F16_SCALE_U * F16_SCALE_LOW;
+            if (storage == MRLBM_F16U && nm == 11 && k == nm + 3) s = F16_SCALE_LOW;
         }
         scale[k] = s;
         iscale[k] = 1.0f / s;
@@ -358,6 +359,7 @@ mrlbm_status mrlbm::domain_alloc(mrlbm_domain* dom)
         dom->lz_t[k] = choose_lz(dom, tile_rows_of_kind(k));
         dom->lz_o[k] = choose_lz_overlap(dom, tile_rows_of_kind(k));
     }
+    dom->lz_s = choose_lz_sums(dom);
     return MRLBM_OK;
 }
 
@@ -403,6 +405,24 @@ int mrlbm::choose_lz_overlap(const mrlbm_domain* dom, int ty)
         if (cols * ((d.nz + lz - 1) / lz) >= 3 * slots) return lz > plain ? lz : plain;
     }
     return plain;
+}
+
+// z planes per CTA of the sums march: 32 where that gives at least 1.4 waves
+// of CTAs, else the longest chunk that does, but not under 8.  Longer chunks
+// save their two lead planes (6 % at 32), but neighbouring columns then drift
+// apart and re-read their halo rows from DRAM instead of L2, and a step of few
+// tiles waits for whole columns.  Measured (one domain alone, us a step):
+// 256^3 FP32 24 / 32 / 43 / 64 / 128 planes 279 / 274 / 283 / 327 / 379;
+// 512^3 FP16 64 / 256 planes 1,745 / 2,519; 128^3 FP32 13 / 16 / 20 / 32
+// planes 41.5 / 45.2 / 47.4 / 61.7.
+int mrlbm::choose_lz_sums(const mrlbm_domain* dom)
+{
+    const mrlbm_desc& d = dom->d;
+    const long long cols = (long long)((d.nx + TILE_X - 1) / TILE_X) * ((d.ny + TYI_BULK - 1) / TYI_BULK);
+    const long long slots = (long long)dom->nsm * SUM_CTAS;
+    int lz = std::min(d.nz, 32);
+    while (lz > 8 && 5 * cols * ((d.nz + lz - 1) / lz) < 7 * slots) lz--;
+    return lz;
 }
 
 bool mrlbm::tile_ordered(const mrlbm_domain* dom, int flags)
@@ -698,7 +718,10 @@ void mrlbm::fill_step_args(const mrlbm_domain* dom, StepArgs& a, int parity, int
     if (dom->has_outflow) flags |= F_OUTFLOW;
     if (d.storage == MRLBM_F16U) flags |= F_SPLITU;
     const int kind = tile_kind(tile_rows(flags));
-    a.lz = dom->lz > 0 ? dom->lz : tile_ordered(dom, flags) ? dom->lz_o[kind] : dom->lz_t[kind];
+    a.lz = dom->lz > 0                 ? dom->lz
+           : sums_march(dom->q, flags) ? dom->lz_s
+           : tile_ordered(dom, flags)  ? dom->lz_o[kind]
+                                       : dom->lz_t[kind];
 }
 
 // Tile-ordered steps (zmarch_step, tile_order_begin): the state is sized and

@@ -15,10 +15,10 @@ template <int Q, typename T, int FLAGS, typename BCP = table_policy_t<Q, FLAGS>>
 static mrlbm_status launch_step_t(const CUtensorMap* maps, const StepArgs& a, cudaStream_t s, bool pdl)
 {
     constexpr int TYI = tile_rows(FLAGS);
-    constexpr int NW = TYI + 2;
+    constexpr int NW = step_warps(Q, FLAGS, TYI);
     const CUtensorMap& map = maps[tile_kind(TYI)];
     constexpr size_t smem = step_smem_bytes<Q, T, FLAGS, TYI, BCP>();
-    static_assert(smem <= smem_budget(TYI), "shared memory over the sm_100 limit");
+    static_assert(smem <= smem_share(step_ctas(Q, FLAGS, TYI)), "shared memory over the sm_100 limit");
     auto kern = zmarch_step<Q, T, FLAGS, TYI, BCP>;
     int dev = 0;
     cudaGetDevice(&dev);
