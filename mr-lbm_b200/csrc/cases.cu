@@ -97,7 +97,7 @@ extern "C" mrlbm_status mrlbm_bc_class_info(int lattice, int bc_matrix_q, uint32
     BcClass c;
     mrlbm_status st = build_bc_class(lattice, mq, node_type, bc_velocity, omega0, &c);
     if (st) return st;
-    memcpy(out, c.ainv, 49 * sizeof(float));
+    for (int r = 0; r < 7; r++) memcpy(out + 7 * r, c.ainv[r], 7 * sizeof(float));
     memcpy(out + 49, c.v, 7 * sizeof(float));
     memcpy(out + 56, c.qa, 7 * sizeof(float));
     out[63] = c.s;

@@ -71,9 +71,16 @@ namespace mrlbm {
 mrlbm_status fail(mrlbm_status st, const char* fmt, ...);
 uint32_t known_mask(int q, uint32_t octants);
 mrlbm_status build_bc_class(int q, int mq, uint32_t word, const double uvel[4][3], double omega0, BcClass* out);
+// geom: the domain's shape and the populations of its resting ghost shell, for
+// the classes that take the total sums (BC_TOTALS); null: none does
+struct WallGeom {
+    int nx, ny, nz;
+    bool wall_x, wall_y;   // not periodic
+    double fext[27];
+};
 mrlbm_status classify_nodes(int q, int mq, const uint32_t* nt, long long n, const double uvel[4][3], double omega0,
                             std::vector<uint8_t>& cls, std::vector<BcClass>& table, bool& any_bc,
-                            bool case_mode = false, const double* t_wall = nullptr);
+                            bool case_mode = false, const double* t_wall = nullptr, const WallGeom* geom = nullptr);
 void storage_scales(int storage, int nm, float* scale, float* iscale);
 // storages kept as fp16 words (plain, or with split velocity)
 inline bool is_half_storage(int storage) { return storage == MRLBM_F16 || storage == MRLBM_F16U; }

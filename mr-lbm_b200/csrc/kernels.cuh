@@ -165,21 +165,31 @@ __device__ __forceinline__ bool smem_ok(const void* p, int bytes, int kind)
 // in X = (rho, rho*Pi).  Its matrix is A(w) = A(w0) + (w - w0) e0 q^T, so the
 // host stores Ainv = A(w0)^-1, v = Ainv e0, qa = q^T Ainv, s = q^T Ainv e0 and
 // the device applies Sherman-Morrison for a per-node omega.
-// 72 words, 16-byte aligned, so the kernel can read a class with vector loads.
+// Rows of 8 words, so the kernel reads the matrix with 16-byte loads (14 for
+// the 49 words); 84 words a class: the lanes of a warp that hold different
+// classes (scattered obstacles) then read a row from different shared-memory
+// banks (21 16-byte words is odd), where 72 words put them 8 to a bank.
+// BC_TOTALS marks a class whose nodes lie on x and y faces of the domain only
+// so that every unknown population would come from outside it, where the ghost
+// shell rests: there the sums over all populations, which every node forms
+// anyway, are the known sums plus constants, and the class carries
+// xc = -A(w0)^-1 (those constants) instead of the kernel selecting populations.
+constexpr uint32_t BC_TOTALS = 1u << 31;
 struct alignas(16) BcClass {
-    float ainv[49];
-    float v[7];
-    float qa[7];
+    float ainv[7][8];  // row r of A(w0)^-1 (7 words), then word r of xc
+    float qa[7];       // q^T A(w0)^-1
     float s;
+    float v[8];        // A(w0)^-1 e0 (7 words), then q^T A(w0)^-1 on the constant part
     float u[3];        // prescribed wall velocity (unscaled)
-    uint32_t known;    // bit i: population i is known (incoming from fluid)
+    uint32_t known;    // bit i: population i is known (incoming from fluid); bit 31: BC_TOTALS
     uint32_t valid;
     uint32_t word;     // the node-type word of the class (nodeTypeMap encoding)
     uint32_t trule;    // thermal rule (bits 0-1), wall normal axis (bits 2-3, 3 = none),
                        // solid side of the normal (bit 4: + side), BC kind (bits 8-10)
     float twall;       // thermal wall value
+    uint32_t pad[4];
 };
-static_assert(sizeof(BcClass) == 288, "BcClass is read as float4 words");
+static_assert(sizeof(BcClass) == 336, "BcClass is read as float4 words");
 
 struct StepArgs {
     void* __restrict__ m_out;         // padded planes [nm][nz+2][ny+2][pitch]
@@ -421,9 +431,7 @@ __device__ __forceinline__ void bc_known_sums(uint32_t known, const float* p, fl
 // mac = rho, u (unscaled), Pi_hat (unscaled xx,xy,xz,yy,yz,zz) from the
 // known-set moment system of class c (the wall-node closed forms of the
 // reference's bc_definition.inc, e.g. src/cases/lidDrivenCavity_3D/
-// bc_definition.inc:637-663, solved generically).  The class words are read
-// one at a time: read as 16-byte vectors they all issue up front and spill at
-// the 102 registers a thread of the two-CTA wall kernels may use.
+// bc_definition.inc:637-663, solved generically).
 template <bool SH>
 __device__ __forceinline__ float class_word(const float* w)
 {
@@ -437,31 +445,65 @@ __device__ __forceinline__ uint32_t class_word(const uint32_t* w)
     else return __ldg(w);
 }
 
+// eight words of a class (a row)
+template <bool SH>
+__device__ __forceinline__ void class_row(const float* w, float (&r)[8])
+{
+    const float4* p = reinterpret_cast<const float4*>(w);
+    float4 x, y;
+    if constexpr (SH) { x = p[0]; y = p[1]; }
+    else { x = __ldg(p); y = __ldg(p + 1); }
+    r[0] = x.x; r[1] = x.y; r[2] = x.z; r[3] = x.w;
+    r[4] = y.x; r[5] = y.y; r[6] = y.z; r[7] = y.w;
+}
+
 // SH: plain loads (c may point at the CTA's shared-memory copy of the class),
-// else read-only cache loads from the table in global memory
-template <int Q, bool SH = false>
+// else read-only cache loads from the table in global memory.  VEC: rows in
+// 16-byte loads; in kernels of many sets, or next to another inlined copy of
+// the solve, they spill, so those read a word at a time.  TOT: classes marked
+// BC_TOTALS take the total sums, rho (1, Pi_hat) of the bulk moments that mac
+// holds on entry (the kernels without a staged table; in the others the second
+// way to the sums costs spills: 128^3 D3Q19 cavity +13 %).  XC: the rows' last
+// word is read where no class takes totals either, as the zero it then is (in
+// the kernels with two solves inlined ptxas spills 12 bytes with it, 44 without).
+template <int Q, bool SH = false, bool VEC = false, bool TOT = false, bool XC = TOT>
 __device__ __forceinline__ void bc_moments(const BcClass* __restrict__ c, const float* p, float omega,
                                            float omega0, float* mac)
 {
-    float b[7], X[7];
-    bc_known_sums<Q>(class_word<SH>(&c->known), p, b);
+    float b[7], X[7], w[8];
+    const uint32_t known = class_word<SH>(&c->known);
+    if (TOT && (known & BC_TOTALS)) {
+        b[0] = mac[0];
+#pragma unroll
+        for (int k = 1; k < 7; k++) b[k] = mac[0] * mac[3 + k];
+    } else {
+        bc_known_sums<Q>(known, p, b);
+    }
 #pragma unroll
     for (int r = 0; r < 7; r++) {
-        float acc = 0.f;
+        if constexpr (VEC) {
+            class_row<SH>(c->ainv[r], w);
+        } else {
 #pragma unroll
-        for (int k = 0; k < 7; k++) acc = fmaf(class_word<SH>(&c->ainv[r * 7 + k]), b[k], acc);
+            for (int k = 0; k < (XC ? 8 : 7); k++) w[k] = class_word<SH>(&c->ainv[r][k]);
+        }
+        float acc = XC ? w[7] : 0.f;   // 0 in classes that take no totals
+#pragma unroll
+        for (int k = 0; k < 7; k++) acc = fmaf(w[k], b[k], acc);
         X[r] = acc;
     }
     // per-node omega (non-Newtonian): Sherman-Morrison update of A(omega0)^-1;
     // a Newtonian domain (omega == omega0) reads none of its words
     const float dw = omega - omega0;
     if (dw != 0.f) {
-        float dot = 0.f;
+        float dot = TOT ? class_word<SH>(&c->v[7]) : 0.f;
+        if constexpr (VEC) class_row<SH>(c->qa, w);
 #pragma unroll
-        for (int r = 0; r < 7; r++) dot = fmaf(class_word<SH>(&c->qa[r]), b[r], dot);
-        const float corr = dw * dot / (1.0f + dw * class_word<SH>(&c->s));
+        for (int r = 0; r < 7; r++) dot = fmaf(VEC ? w[r] : class_word<SH>(&c->qa[r]), b[r], dot);
+        const float corr = dw * dot / (1.0f + dw * (VEC ? w[7] : class_word<SH>(&c->s)));
+        if constexpr (VEC) class_row<SH>(c->v, w);
 #pragma unroll
-        for (int r = 0; r < 7; r++) X[r] = fmaf(-corr, class_word<SH>(&c->v[r]), X[r]);
+        for (int r = 0; r < 7; r++) X[r] = fmaf(-corr, VEC ? w[r] : class_word<SH>(&c->v[r]), X[r]);
     }
     const float rho = X[0], ir = 1.0f / rho;
     mac[0] = rho;
@@ -544,7 +586,7 @@ struct TableBC {
     static __device__ __forceinline__ void apply(const StepArgs& a, uint8_t cls, const float* p, float omega,
                                                  int x, int y, int z, float* mac)
     {
-        bc_moments<Q>(a.bc + cls, p, omega, a.omega0, mac);
+        bc_moments<Q, false, false, true>(a.bc + cls, p, omega, a.omega0, mac);
     }
     // C and 3 sum g c at a thermal boundary node: the class's run-time rule
     template <typename T>
@@ -563,7 +605,7 @@ struct OutflowBC {
         const BcClass* c = a.bc + cls;
         const uint32_t kw = __ldg(&c->trule);
         if (((kw >> 8) & 7u) == BC_KIND_OUTFLOW) outflow_moments<T>(a, kw, x, y, z, mac);
-        else bc_moments<Q>(c, p, omega, a.omega0, mac);
+        else bc_moments<Q, false, false, true>(c, p, omega, a.omega0, mac);
     }
     template <typename T>
     static __device__ __forceinline__ void thermal(const StepArgs& a, uint8_t cls, const float* pg, unsigned oidx,
@@ -582,21 +624,27 @@ struct TableBCShared : TableBC {
     static __device__ __forceinline__ void apply(const StepArgs& a, uint8_t cls, const float* p, float omega,
                                                  int x, int y, int z, float* mac)
     {
-        if ((int)cls < staged_classes()) bc_moments<Q, true>(staged_class(cls), p, omega, a.omega0, mac);
-        else bc_moments<Q>(a.bc + cls, p, omega, a.omega0, mac);
+        if ((int)cls < staged_classes()) bc_moments<Q, true, false, false, true>(staged_class(cls), p, omega, a.omega0, mac);
+        else bc_moments<Q, false, false, false, true>(a.bc + cls, p, omega, a.omega0, mac);
     }
 };
 
-// The class table staged in shared memory, for the non-Newtonian D3Q19 wall
-// kernels: one solve through a generic pointer to the shared or the global
-// copy (two copies spill there; +7 % on a power-law duct against TableBC).
+// The class table staged in shared memory, one solve through a generic pointer
+// to the shared or the global copy.  For the non-Newtonian D3Q19 wall kernels
+// (VEC; two copies spill there) and the D3Q19 batches, whose kernel holds every
+// flag set and would spill with rows of 16 bytes).  Measured on a 128^3
+// power-law duct with 5 % scattered obstacles, three quarters of its nodes at
+// walls: rows in 16-byte loads and 84-word classes 115 us a step against 176
+// with single words of 72-word classes, whose lanes met 8 to a bank; 109 with
+// the table in the order of use.
+template <bool VEC>
 struct TableBCGeneric : TableBC {
     template <int Q, typename T>
     static __device__ __forceinline__ void apply(const StepArgs& a, uint8_t cls, const float* p, float omega,
                                                  int x, int y, int z, float* mac)
     {
         const BcClass* c = (int)cls < staged_classes() ? staged_class(cls) : a.bc + cls;
-        bc_moments<Q, true>(c, p, omega, a.omega0, mac);
+        bc_moments<Q, true, VEC>(c, p, omega, a.omega0, mac);
     }
 };
 
@@ -605,14 +653,14 @@ template <typename BCP>
 struct stages_classes : std::false_type {};
 template <>
 struct stages_classes<TableBCShared> : std::true_type {};
-template <>
-struct stages_classes<TableBCGeneric> : std::true_type {};
+template <bool VEC>
+struct stages_classes<TableBCGeneric<VEC>> : std::true_type {};
 
 // the class-table policy of a single-domain wall kernel
 template <int Q, int FLAGS>
 using table_policy_t =
     std::conditional_t<Q == 19 && (FLAGS & F_THERMAL) == 0,
-                       std::conditional_t<(FLAGS & (F_POWERLAW | F_BINGHAM)) != 0, TableBCGeneric, TableBCShared>,
+                       std::conditional_t<(FLAGS & (F_POWERLAW | F_BINGHAM)) != 0, TableBCGeneric<true>, TableBCShared>,
                        TableBC>;
 
 // Power-law omega by Newton iteration (src/nnf.h:61-89 with its compile
@@ -1359,7 +1407,11 @@ struct ZSmem {
     static constexpr size_t fixed = 128 + ex_bytes + edge_bytes;
     // RESERVE: the kernel's static shared memory, which the CTA's share holds too
     static constexpr size_t budget = smem_budget(TYI) - RESERVE;
-    static constexpr int NS = fixed + NSTAGE_MAX * stage_max <= budget         ? NSTAGE_MAX
+    // (walls of six or more pairs, the non-Newtonian and split sets, take 3: a duct of obstacles
+    // gains more from 90 staged classes than from the fourth stage, where 39
+    // fit: 128^3 102 us a step against 109, split fp16 7.7 ms against 7.9)
+    static constexpr int NS = WC && NPM >= 6 && RESERVE == 0                   ? NSTAGE_MAX - 1
+                              : fixed + NSTAGE_MAX * stage_max <= budget       ? NSTAGE_MAX
                               : fixed + (NSTAGE_MAX - 1) * stage_max <= budget ? NSTAGE_MAX - 1
                                                                                : NSTAGE_MAX - 2;
     static constexpr size_t ring_bytes = fixed + NS * stage_max;

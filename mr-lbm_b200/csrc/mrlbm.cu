@@ -180,7 +180,7 @@ mrlbm_status mrlbm::build_bc_class(int q, int mq, uint32_t word, const double uv
     }
     memset(out, 0, sizeof(*out));
     for (int rr = 0; rr < 7; rr++)
-        for (int c = 0; c < 7; c++) out->ainv[rr * 7 + c] = (float)inv[rr][c];
+        for (int c = 0; c < 7; c++) out->ainv[rr][c] = (float)inv[rr][c];
     for (int rr = 0; rr < 7; rr++) {
         out->v[rr] = (float)inv[rr][0];
         out->qa[rr] = (float)qa[rr];
@@ -508,15 +508,88 @@ static mrlbm_status thermal_rule_of(uint32_t word, const double t_wall[4], BcCla
     return MRLBM_OK;
 }
 
+// Whether every unknown population of a node at x, y (known: the known ones) would
+// come from outside a non-periodic x or y axis.  (Not z: a slab of a cut
+// domain has neighbours there.)
+static bool takes_totals(const WallGeom& g, int q, uint32_t known, int x, int y)
+{
+    for (int i = 0; i < q; i++) {
+        if ((known >> i) & 1u) continue;
+        const int sx = x - lat_cx(i), sy = y - lat_cy(i);
+        if (!((g.wall_x && (sx < 0 || sx >= g.nx)) || (g.wall_y && (sy < 0 || sy >= g.ny)))) return false;
+    }
+    return true;
+}
+
+// The constants of a class that takes the total sums: minus its solve of the
+// ghost shell's populations in its unknown directions.
+static void set_totals(const WallGeom& g, int q, BcClass* c)
+{
+    double bu[7] = {};
+    for (int i = 0; i < q; i++) {
+        if ((c->known >> i) & 1u) continue;
+        double h[6], gg[6];
+        hg(i, h, gg);
+        bu[0] += g.fext[i];
+        for (int k = 0; k < 6; k++) bu[1 + k] += g.fext[i] * h[k];
+    }
+    double qc = 0.0;
+    for (int r = 0; r < 7; r++) {
+        double x = 0.0;
+        for (int k = 0; k < 7; k++) x -= (double)c->ainv[r][k] * bu[k];
+        c->ainv[r][7] = (float)x;
+        qc -= (double)c->qa[r] * bu[r];
+    }
+    c->v[7] = (float)qc;
+    c->known |= BC_TOTALS;
+}
+
+// a moment of the ghost shell as the step reads it (the storage's rounding)
+static double stored_value(const mrlbm_domain* dom, int m)
+{
+    const float v = dom->ext[m], s = dom->scale[m];
+    if (dom->d.storage == MRLBM_F32) return v;
+    if (is_half_storage(dom->d.storage)) return (double)__half2float(__float2half_rn(v * s)) / s;
+    return (double)__bfloat162float(__float2bfloat16_rn(v * s)) / s;
+}
+
+static WallGeom wall_geom(const mrlbm_domain* dom)
+{
+    const mrlbm_desc& d = dom->d;
+    WallGeom g{d.nx, d.ny, d.nz, !d.periodic[0], !d.periodic[1], {}};
+    double m[10];
+    for (int k = 0; k < 10; k++) m[k] = stored_value(dom, k);
+    for (int i = 0; i < dom->q; i++) {
+        const double cx = lat_cx(i), cy = lat_cy(i), cz = lat_cz(i);
+        g.fext[i] = (d.rho0 + m[0]) * lat_w(dom->q, i) *
+                    (1.0 - (m[4] + m[7] + m[9]) / 3.0 + cx * m[1] + cy * m[2] + cz * m[3] + cx * cx * m[4] +
+                     cy * cy * m[7] + cz * cz * m[9] + cx * cy * m[5] + cx * cz * m[6] + cy * cz * m[8]);
+    }
+    return g;
+}
+
 mrlbm_status mrlbm::classify_nodes(int q, int mq, const uint32_t* nt, long long n, const double uvel[4][3],
                                    double omega0, std::vector<uint8_t>& cls, std::vector<BcClass>& table,
-                                   bool& any_bc, bool case_mode, const double* t_wall)
+                                   bool& any_bc, bool case_mode, const double* t_wall, const WallGeom* geom)
 {
-    std::map<uint32_t, int> ids;
+    // class of a node type: a run-time key (octant mask, BC kind, velocity
+    // index, thermal bits, total sums or not) indexes a table, a case's whole
+    // word a map
+    const uint32_t key_bits = t_wall ? 0x1FFFFu : 0x1FFFu, TOTALS_KEY = key_bits + 1;
+    std::vector<int16_t> ids(case_mode ? 0 : 2 * TOTALS_KEY, (int16_t)-1);
+    std::map<uint32_t, int> case_ids;
+    // whether a node takes the total sums depends on its mask and on which of
+    // the x and y faces it lies on only: -1 not worked out yet
+    std::vector<int8_t> totals_of(geom ? 256 * 16 : 0, (int8_t)-1);
+    int x = -1, y = 0;
     table.assign(1, BcClass{});  // class 0: bulk (unused entry)
     cls.resize(n);
     any_bc = false;
     for (long long k = 0; k < n; k++) {
+        if (geom && ++x == geom->nx) {
+            x = 0;
+            if (++y == geom->ny) y = 0;
+        }
         const uint32_t w = nt[k];
         // run-time classes key on the octant mask, BC kind and velocity index;
         // case mode hands the whole word to the case's own snippet (like the
@@ -527,10 +600,28 @@ mrlbm_status mrlbm::classify_nodes(int q, int mq, const uint32_t* nt, long long 
         any_bc = true;
         if (solid) { cls[k] = CLS_SOLID; continue; }
         // (thermal domains also key on the thermal rule and value index)
-        const uint32_t key = case_mode ? w : (w & (t_wall ? 0x1FFFFu : 0x1FFFu));
-        auto it = ids.find(key);
-        if (it == ids.end()) {
-            if ((int)table.size() >= 255) return fail(MRLBM_EINVAL, "more than 254 distinct boundary node types");
+        const uint32_t key = case_mode ? w : (w & key_bits);
+        bool totals = false;
+        if (geom && ((w >> 8) & 7u) != 2u) {
+            const int face = (x == 0) | (x == geom->nx - 1) << 1 | (y == 0) << 2 | (y == geom->ny - 1) << 3;
+            int8_t& t = totals_of[(w & 0xFFu) * 16 + face];
+            if (t < 0) t = takes_totals(*geom, q, known_mask(q, w & 0xFFu), x, y);
+            totals = t != 0;
+        }
+        int id;
+        if (case_mode) {
+            auto it = case_ids.find(key);
+            id = it == case_ids.end() ? -1 : it->second;
+        } else {
+            id = ids[key | (totals ? TOTALS_KEY : 0u)];
+        }
+        if (id < 0) {
+            if ((int)table.size() >= 255) {
+                // two classes of a node type (with and without total sums)
+                // may not cost a domain its room in the table
+                if (geom) return classify_nodes(q, mq, nt, n, uvel, omega0, cls, table, any_bc, case_mode, t_wall, nullptr);
+                return fail(MRLBM_EINVAL, "more than 254 distinct boundary node types");
+            }
             BcClass c;
             memset(&c, 0, sizeof(c));
             c.word = key;
@@ -539,11 +630,34 @@ mrlbm_status mrlbm::classify_nodes(int q, int mq, const uint32_t* nt, long long 
             c.word = key;
             if (!case_mode && (st = class_normal(key, &c))) return st;
             if (t_wall && !case_mode && (st = thermal_rule_of(key, t_wall, &c))) return st;
-            const int id = (int)table.size();
+            if (totals) set_totals(*geom, q, &c);
+            id = (int)table.size();
             table.push_back(c);
-            it = ids.emplace(key, id).first;
+            if (case_mode) case_ids.emplace(key, id);
+            else ids[key | (totals ? TOTALS_KEY : 0u)] = (int16_t)id;
         }
-        cls[k] = (uint8_t)it->second;
+        cls[k] = (uint8_t)id;
+    }
+    // The wall kernels stage the first classes of the table in shared memory:
+    // put those of the most nodes first (a duct of scattered obstacles has all
+    // 254 masks, of which a few dozen cover most nodes).  Every kernel holds 37
+    // classes at least, so a smaller table needs no order.
+    if (table.size() > 37) {
+        long long count[256] = {};
+        for (long long k = 0; k < n; k++) count[cls[k]]++;
+        std::vector<int> order(table.size() - 1);
+        for (size_t i = 0; i < order.size(); i++) order[i] = (int)i + 1;
+        std::stable_sort(order.begin(), order.end(), [&](int u, int v) { return count[u] > count[v]; });
+        uint8_t to[256];
+        for (int i = 0; i < 256; i++) to[i] = (uint8_t)i;
+        std::vector<BcClass> sorted(table.size());
+        sorted[0] = table[0];
+        for (size_t i = 0; i < order.size(); i++) {
+            sorted[i + 1] = table[order[i]];
+            to[order[i]] = (uint8_t)(i + 1);
+        }
+        table.swap(sorted);
+        for (long long k = 0; k < n; k++) cls[k] = to[cls[k]];
     }
     return MRLBM_OK;
 }
@@ -556,9 +670,12 @@ static mrlbm_status set_node_types_impl(mrlbm_domain* dom, const uint32_t* nt, b
     std::vector<uint8_t> cls;
     std::vector<BcClass> table;
     bool any = false;
+    // the sets whose kernels take total sums (bc_moments' TOT)
+    const bool totals = !case_mode && (dom->q == 27 || d.thermal);
+    const WallGeom geom = wall_geom(dom);
     mrlbm_status st =
         classify_nodes(dom->q, d.bc_matrix_q, nt, n, d.bc_velocity, dom->omega0, cls, table, any, case_mode,
-                       d.thermal ? d.t_wall : nullptr);
+                       d.thermal ? d.t_wall : nullptr, totals ? &geom : nullptr);
     if (st) return st;
     bool outflow = false;
     for (const BcClass& c : table)

@@ -63,3 +63,61 @@ def test_d3q27_16bit(shape, storage, ulp):
     # split storage keeps the second moments (and the little they give u) in one fp16 word
     assert low < STEPS * max(ulp, 2.0 ** -14 if storage == mrlbm.F16U else 0.0), low
     assert second < 4 * STEPS * max(ulp, 2.0 ** -11), second
+
+
+# ---- walls that take the total sums (x and y faces) and the class table's order
+
+WALL_LOW, WALL_SECOND = 2e-5, 3e-4   # whole populations: eps / u^2 on the second moments, as in test_gpu_parity
+
+
+def wall_errors(d, nt):
+    low, second = errors(d, 0, nt)
+    return low, second
+
+
+@pytest.mark.parametrize("shape", [(33, 9, 5), (32, 8, 4), (5, 40, 6), (31, 7, 3)])
+def test_d3q27_cavity(shape):
+    nx, ny, nz = shape
+    d = mrlbm.lid_cavity_desc(nx, re=20.0, lid_u=0.05, lattice=mrlbm.D3Q27, ny=ny, nz=nz)
+    low, second = wall_errors(d, mrlbm.lid_cavity_node_types(nx, ny, nz, 1))
+    assert low < WALL_LOW and second < WALL_SECOND, (low, second)
+
+
+@pytest.mark.parametrize("storage,tol", [(mrlbm.F16, 2.0 ** -11), (mrlbm.BF16, 2.0 ** -8), (mrlbm.F16U, 2.0 ** -11)])
+def test_d3q27_cavity_16bit(storage, tol):
+    """The ghost shell's moments are subtracted as the storage rounds them."""
+    nx, ny, nz = 33, 17, 9
+    d = mrlbm.lid_cavity_desc(nx, re=20.0, lid_u=0.05, lattice=mrlbm.D3Q27, storage=storage, ny=ny, nz=nz)
+    low, second = wall_errors(d, mrlbm.lid_cavity_node_types(nx, ny, nz, 1))
+    assert low < 4 * STEPS * tol and second < 16 * STEPS * tol, (low, second)
+
+
+@pytest.mark.parametrize("lattice", [mrlbm.D3Q19, mrlbm.D3Q27])
+def test_inner_plane_typed_like_the_face(lattice):
+    """The same node type on the x face (sources outside) and on an inner
+    plane (fluid sources): only the face may take the total sums."""
+    nx, ny, nz = 20, 10, 6
+    nt = np.zeros((nz, ny, nx), dtype=np.uint32)
+    nt[:, :, 0] = mrlbm.WEST
+    nt[:, :, 11] = mrlbm.WEST
+    nt[:, :, -1] = mrlbm.EAST
+    d = mrlbm.make_desc(nx, ny, nz, lattice=lattice, periodic=(0, 1, 1), tau=0.7)
+    low, second = wall_errors(d, nt)
+    assert low < WALL_LOW and second < WALL_SECOND, (low, second)
+
+
+@pytest.mark.parametrize("lattice", [mrlbm.D3Q19, mrlbm.D3Q27])
+@pytest.mark.parametrize("rheology", [mrlbm.NEWTONIAN, mrlbm.POWERLAW])
+@pytest.mark.parametrize("fill", [0.02, 0.3])
+def test_scattered_obstacles(lattice, rheology, fill):
+    """Few and (nearly) all of the 254 masks: the table in order of use, staged
+    and past the staged classes."""
+    nx, ny, nz = 34, 17, 12
+    rng = np.random.default_rng(3)
+    solid = np.zeros((nz, ny, nx), dtype=np.uint8)
+    solid[:, 1:-1, 1:-1] = rng.random((nz, ny - 2, nx - 2)) < fill
+    nt = mrlbm.voxel_node_types(solid, (0, 0, 1))
+    d = mrlbm.make_desc(nx, ny, nz, lattice=lattice, periodic=(0, 0, 1), tau=0.8, force=(0, 0, 2e-5), rheology=rheology,
+                        nnf_n=0.9)
+    low, second = wall_errors(d, nt)
+    assert low < 2 * WALL_LOW and second < 2 * WALL_SECOND, (low, second)
