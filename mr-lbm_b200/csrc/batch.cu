@@ -113,13 +113,14 @@ int batch_flags(const mrlbm_domain* dom)
     StepArgs a;
     int flags;
     fill_step_args(dom, a, 0, flags);
-    if (flags & (F_FORCE | F_POWERLAW | F_BINGHAM)) flags |= F_BC;
+    flags &= ~F_DENSE;   // a launch shape of the single-domain step
+    if (flags & (F_FORCE | F_POWERLAW | F_BINGHAM)) flags = (flags & ~F_SUMS) | F_BC;
     return flags;
 }
 
 bool flags_supported(int f)
 {
-    f &= ~F_SPLITU;  // every set below also with split-velocity storage
+    f &= ~(F_SPLITU | F_SUMS);  // every set below also with split-velocity storage, or in the sums march
     return f == 0 || f == F_BC || f == (F_BC | F_FORCE) || f == (F_BC | F_FORCE | F_POWERLAW);
 }
 

@@ -46,6 +46,8 @@ struct mrlbm_domain {
     int lz_t[2] = {16, 16};          // single-domain z planes per CTA, per tile kind
     int lz_o[2] = {16, 16};          // the same for tile-ordered (overlapping) steps
     int lz_s = 16;                   // the same for the sums march
+    bool dense = false, sums = false;   // dense_domain, sums_domain
+    int lz_b[2] = {16, 16};          // z planes per CTA of F_DENSE sets: whole launches, tile-ordered
     int nsm = 148;                   // SMs of the device the domain lives on
     cudaStream_t stream = nullptr;      // where the domain's work is queued
     cudaStream_t own_stream = nullptr;  // the stream the domain created (stream unless mrlbm_set_stream)
@@ -85,8 +87,8 @@ void storage_scales(int storage, int nm, float* scale, float* iscale);
 // storages kept as fp16 words (plain, or with split velocity)
 inline bool is_half_storage(int storage) { return storage == MRLBM_F16 || storage == MRLBM_F16U; }
 mrlbm_status domain_alloc(mrlbm_domain* dom);
-int choose_lz(const mrlbm_domain* dom, int tyi);
-int choose_lz_overlap(const mrlbm_domain* dom, int tyi);
+int choose_lz(const mrlbm_domain* dom, int tyi, int ctas);
+int choose_lz_overlap(const mrlbm_domain* dom, int tyi, int ctas);
 int choose_lz_sums(const mrlbm_domain* dom);
 // whether a step with these flags is tile-ordered (overlapping launches)
 bool tile_ordered(const mrlbm_domain* dom, int flags);

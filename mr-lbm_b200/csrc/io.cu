@@ -377,7 +377,7 @@ extern "C" mrlbm_status mrlbm_save_info(mrlbm_domain* dom, const char* path_file
     StepArgs sa;
     int flags = 0;
     fill_step_args(dom, sa, dom->cur, flags);
-    // the nominal tile of the flag set (the sums march has a z chunk of its own), as in mrlbm_info_text
+    // the nominal tile of the flag set (the bulk sets have z chunks of their own), as in mrlbm_info_text
     const int kind = tile_kind(tile_rows(flags));
     const int lz = dom->lz > 0 ? dom->lz : tile_ordered(dom, flags) ? dom->lz_o[kind] : dom->lz_t[kind];
     const std::string t = info_text(dom->d, id_sim, case_name, nsteps, mlups, tile_rows(flags), lz);
@@ -396,7 +396,7 @@ extern "C" mrlbm_status mrlbm_info_text(const mrlbm_desc* d, const char* id_sim,
     tmp.nsm = 148;
     const int flags = (d->rheology != MRLBM_NEWTONIAN ? F_POWERLAW | F_BC : 0) | (d->thermal ? F_THERMAL : 0);
     const int by = tile_rows(flags);
-    const int lz = tile_ordered(&tmp, flags) ? choose_lz_overlap(&tmp, by) : choose_lz(&tmp, by);
+    const int lz = tile_ordered(&tmp, flags) ? choose_lz_overlap(&tmp, by, ctas_per_sm(by)) : choose_lz(&tmp, by, ctas_per_sm(by));
     const std::string t = info_text(*d, id_sim, case_name, nsteps, mlups, by, lz);
     *len = t.size();
     if (buf) {

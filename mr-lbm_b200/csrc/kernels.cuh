@@ -17,11 +17,12 @@
 //     the shell equal to the wrapped interior: the kernel writes the extra
 //     copies of boundary nodes.  Wall axes keep the shell at the exterior rest
 //     state.  So every halo read is an in-bounds tile read with no wrap logic.
-//   * A CTA owns a column of 30 x TYI interior nodes in (x, y) and a chunk of
-//     LZ planes in z.  Warp w holds row y = Y0 - 1 + w, lane l holds
-//     x = X0 - 1 + l: the outer lanes / warps are the one-node halo.
-//   * One elected thread streams the planes of the column into a 4-stage
-//     shared-memory ring with cp.async.bulk.tensor (TMA) and mbarrier
+//   * A CTA owns a column of 32 x TYI interior nodes in (x, y) and a chunk of
+//     LZ planes in z.  Warp w < TYI holds row y = Y0 + w, lane l holds
+//     x = X0 + l; two helper warps produce only the populations that enter
+//     the column from the ring of nodes around it.
+//   * One elected thread streams the planes of the column into a ring of two
+//     to four stages in shared memory with cp.async.bulk.tensor (TMA) and mbarrier
 //     transaction counts; the waits are bounded and a timeout makes every
 //     thread leave together with an error flag set.
 //   * Each production step reconstructs the post-collision populations of
@@ -59,6 +60,8 @@ enum : int {
     F_THERMAL = 16,  // thermal scalar C on D3G19 (4 more stored moments, Boussinesq force)
     F_OUTFLOW = 32,  // some wall class is an outflow (selects the OutflowBC policy at launch)
     F_SPLITU = 64,   // 16-bit storage with each velocity component split in a high and a low word
+    F_DENSE = 128,   // D3Q19 bulk sets at three CTAs an SM (set at launch for large domains)
+    F_SUMS = 256,    // D3Q27 bulk sets in the sums march (set at launch, sums_domain)
 };
 
 // most stored moments per node: 10 flow moments + omega, or + C and its flux
@@ -109,10 +112,7 @@ __host__ __device__ constexpr int nmoments_of(int flags)
 }
 __host__ __device__ constexpr int npairs_of(int flags) { return (nmoments_of(flags) + 1) / 2; }
 // flag sets of the sums march (sum_march.cuh)
-__host__ __device__ constexpr bool sums_march(int q, int flags)
-{
-    return q == 27 && (flags & ~(F_FORCE | F_SPLITU)) == 0;
-}
+__host__ __device__ constexpr bool sums_march(int q, int flags) { return q == 27 && (flags & F_SUMS) != 0; }
 // index of a tile height among the domain's tensor maps and z chunks
 __host__ __device__ constexpr int tile_kind(int tyi) { return tyi == TYI_BULK ? 0 : 1; }
 __host__ __device__ constexpr int tile_rows_of_kind(int kind) { return kind == 0 ? TYI_BULK : TYI_WALL; }
@@ -1393,7 +1393,8 @@ __device__ __forceinline__ void prod_b(const StepArgs& a, int k, int zp, const f
 // (kernels that switch between flag sets at run time size them for the
 // largest set), and the ring has NSTAGE_MAX stages when they fit next to the
 // exchange buffers, else fewer.
-template <int Q, typename T, int TYI, int NPM, bool TH = false, int RESERVE = 0, bool WC = false>
+template <int Q, typename T, int TYI, int NPM, bool TH = false, int RESERVE = 0, bool WC = false,
+          int CTAS = ctas_per_sm(TYI)>
 struct ZSmem {
     static constexpr int NR = TYI + 2;  // stage rows = exchange rows
     static constexpr size_t stage_max = ((size_t)NR * NPM * 2 * box_x<T>() * sizeof(T) + 127) / 128 * 128;
@@ -1406,7 +1407,7 @@ struct ZSmem {
     static constexpr size_t edge_bytes = (size_t)(TH ? 2 : 1) * edge_n * 16;
     static constexpr size_t fixed = 128 + ex_bytes + edge_bytes;
     // RESERVE: the kernel's static shared memory, which the CTA's share holds too
-    static constexpr size_t budget = smem_budget(TYI) - RESERVE;
+    static constexpr size_t budget = smem_share(CTAS) - RESERVE;
     // (walls of six or more pairs, the non-Newtonian and split sets, take 3: a duct of obstacles
     // gains more from 90 staged classes than from the fourth stage, where 39
     // fit: 128^3 102 us a step against 109, split fp16 7.7 ms against 7.9)
@@ -1540,9 +1541,8 @@ struct ZRing {
 // Per-CTA pipeline state of the z-march over one column.  Warps 0 .. TYI-1 run
 // the interior pipeline (interior_loop), warps TYI and TYI+1 the helper one
 // (helper_loop); both take the same barriers in the same order.
-template <int Q, typename T, int FLAGS, int TYI, typename BCP, int NPM, int RES = 0, bool WC = false>
-struct ZMarch : ZRing<T, TYI, npairs_of(FLAGS), ZSmem<Q, T, TYI, NPM, (FLAGS & F_THERMAL) != 0, RES, WC>> {
-    using SM = ZSmem<Q, T, TYI, NPM, (FLAGS & F_THERMAL) != 0, RES, WC>;
+template <int Q, typename T, int FLAGS, int TYI, typename BCP, typename SM>
+struct ZMarch : ZRing<T, TYI, npairs_of(FLAGS), SM> {
     using Ring = ZRing<T, TYI, npairs_of(FLAGS), SM>;
     using Ring::NR;
     using Ring::a;
@@ -1757,18 +1757,16 @@ struct ZMarch : ZRing<T, TYI, npairs_of(FLAGS), ZSmem<Q, T, TYI, NPM, (FLAGS & F
 // One column (X0, Y0) x planes [z0, zend) of one domain.  g0 is the CTA's
 // running production count (advanced by the column's productions).  Returns
 // false when a bounded wait timed out (the CTA must stop).
-template <int Q, typename T, int FLAGS, int TYI, typename BCP = TableBC, int NPM, int RES, bool WC>
+template <int Q, typename T, int FLAGS, int TYI, typename BCP = TableBC, typename SM>
 __device__ __forceinline__ bool zmarch_column(const StepArgs& a, const CUtensorMap* map, int X0, int Y0, int z0,
-                                              int zend,
-                                              const ZSmem<Q, T, TYI, NPM, (FLAGS & F_THERMAL) != 0, RES, WC>& sm,
-                                              unsigned& g0)
+                                              int zend, const SM& sm, unsigned& g0)
 {
-    using ZM = ZMarch<Q, T, FLAGS, TYI, BCP, NPM, RES, WC>;
+    using ZM = ZMarch<Q, T, FLAGS, TYI, BCP, SM>;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     ZM zm(a, map, sm, g0, X0, Y0, z0, zend);
 #ifdef MRLBM_BOUNDS_CHECK
     if (threadIdx.x == 0) {
-        using SMT = ZSmem<Q, T, TYI, NPM, (FLAGS & F_THERMAL) != 0, RES, WC>;
+        using SMT = SM;
         g_bounds.stage_lo = smem_u32(sm.stages);
         g_bounds.stage_hi = smem_u32(sm.stages) + (unsigned)(SMT::NS * SMT::stage_max);
         g_bounds.ex_lo = smem_u32(sm.ex4);
@@ -1914,16 +1912,23 @@ __host__ __device__ constexpr int step_warps(int q, int flags, int tyi)
 {
     return sums_march(q, flags) ? tyi / SUM_ROWS + 1 : tyi + 2;
 }
+// F_DENSE: the D3Q19 bulk sets (five pairs) fit three CTAs an SM with 64
+// registers a thread and a ring of three stages; two CTAs keep 72 and four.
+// Measured (us, among others / alone): ragged 203 x 173 x 121 box, 20 steps,
+// 1,543 / 1,676 against 1,624 / 1,706; 256^3, 10 steps, 2,730 / 2,891 against
+// 2,851 / 2,916.  A domain of few tiles runs alone slower with them (64^3, 50
+// steps, 664 against 561; 128^3 FP16, 20 steps, 789 against 787 at its best
+// chunk), so small ones keep two: dense_domain.
 __host__ __device__ constexpr int step_ctas(int q, int flags, int tyi)
 {
-    return sums_march(q, flags) ? SUM_CTAS : ctas_per_sm(tyi);
+    return sums_march(q, flags) ? SUM_CTAS : (flags & F_DENSE) ? 3 : ctas_per_sm(tyi);
 }
 
 template <int Q, typename T, int FLAGS, int TYI, typename BCP>
 using step_smem_t =
     std::conditional_t<sums_march(Q, FLAGS), SumSmem<T, TYI, npairs_of(FLAGS)>,
                        ZSmem<Q, T, TYI, npairs_of(FLAGS), (FLAGS & F_THERMAL) != 0, 0,
-                             (FLAGS & F_BC) != 0 && stages_classes<BCP>::value>>;
+                             (FLAGS & F_BC) != 0 && stages_classes<BCP>::value, step_ctas(Q, FLAGS, TYI)>>;
 
 // Single-domain step: one CTA per (x tile, y tile, z chunk of lz planes).
 // Launch order runs x tiles fastest, so the CTAs resident at one time march

@@ -285,6 +285,9 @@ extern "C" mrlbm_status mrlbm_domain_bytes(const mrlbm_desc* d, size_t* bytes)
     return MRLBM_OK;
 }
 
+static bool dense_domain(const mrlbm_domain* dom);
+static bool sums_domain(const mrlbm_domain* dom);
+
 mrlbm_status mrlbm::domain_alloc(mrlbm_domain* dom)
 {
     const mrlbm_desc& d = dom->d;
@@ -356,10 +359,15 @@ mrlbm_status mrlbm::domain_alloc(mrlbm_domain* dom)
         dom->nsm = nsm > 0 ? nsm : 148;
     }
     for (int k = 0; k < 2; k++) {
-        dom->lz_t[k] = choose_lz(dom, tile_rows_of_kind(k));
-        dom->lz_o[k] = choose_lz_overlap(dom, tile_rows_of_kind(k));
+        const int ty = tile_rows_of_kind(k);
+        dom->lz_t[k] = choose_lz(dom, ty, ctas_per_sm(ty));
+        dom->lz_o[k] = choose_lz_overlap(dom, ty, ctas_per_sm(ty));
     }
     dom->lz_s = choose_lz_sums(dom);
+    dom->dense = dense_domain(dom);
+    dom->sums = sums_domain(dom);
+    dom->lz_b[0] = choose_lz(dom, TYI_BULK, step_ctas(19, F_DENSE, TYI_BULK));
+    dom->lz_b[1] = choose_lz_overlap(dom, TYI_BULK, step_ctas(19, F_DENSE, TYI_BULK));
     return MRLBM_OK;
 }
 
@@ -367,7 +375,7 @@ mrlbm_status mrlbm::domain_alloc(mrlbm_domain* dom)
 // lz outputs, and the grid runs in ceil(CTAs / SMs) waves, so the step time
 // goes as waves * (lz + 2 + start-up): pick the chunk count that minimises it (the last
 // wave full, few restarts).
-int mrlbm::choose_lz(const mrlbm_domain* dom, int ty)
+int mrlbm::choose_lz(const mrlbm_domain* dom, int ty, int per_sm)
 {
     const mrlbm_desc& d = dom->d;
     const long long cols = (long long)((d.nx + TILE_X - 1) / TILE_X) * ((d.ny + ty - 1) / ty);
@@ -376,7 +384,7 @@ int mrlbm::choose_lz(const mrlbm_domain* dom, int ty)
     for (int nzc = 1; nzc <= d.nz; nzc++) {
         const int lz = (d.nz + nzc - 1) / nzc;
         const long long ctas = cols * ((d.nz + lz - 1) / lz);
-        const long long slots = (long long)dom->nsm * ctas_per_sm(ty);
+        const long long slots = (long long)dom->nsm * per_sm;
         const long long waves = (ctas + slots - 1) / slots;
         const long long cost = waves * (lz + 2 + 3);  // + a CTA start-up of about 3 planes
         if (best_cost < 0 || cost < best_cost) {
@@ -394,12 +402,12 @@ int mrlbm::choose_lz(const mrlbm_domain* dom, int ty)
 // a grid under about three waves of CTAs loses the overlap (a 128^3 cavity
 // ran 37.6 GLUPS at 32 planes, 20.9 at 64).  So: the longest chunk with at
 // least 4 chunks a column and 3 waves of CTAs, if longer than the plain choice.
-int mrlbm::choose_lz_overlap(const mrlbm_domain* dom, int ty)
+int mrlbm::choose_lz_overlap(const mrlbm_domain* dom, int ty, int per_sm)
 {
     const mrlbm_desc& d = dom->d;
-    const int plain = choose_lz(dom, ty);
+    const int plain = choose_lz(dom, ty, per_sm);
     const long long cols = (long long)((d.nx + TILE_X - 1) / TILE_X) * ((d.ny + ty - 1) / ty);
-    const long long slots = (long long)dom->nsm * ctas_per_sm(ty);
+    const long long slots = (long long)dom->nsm * per_sm;
     for (int nzc = 4; nzc <= d.nz; nzc++) {
         const int lz = (d.nz + nzc - 1) / nzc;
         if (cols * ((d.nz + lz - 1) / lz) >= 3 * slots) return lz > plain ? lz : plain;
@@ -407,21 +415,53 @@ int mrlbm::choose_lz_overlap(const mrlbm_domain* dom, int ty)
     return plain;
 }
 
-// z planes per CTA of the sums march: 32 where that gives at least 1.4 waves
-// of CTAs, else the longest chunk that does, but not under 8.  Longer chunks
-// save their two lead planes (6 % at 32), but neighbouring columns then drift
-// apart and re-read their halo rows from DRAM instead of L2, and a step of few
-// tiles waits for whole columns.  Measured (one domain alone, us a step):
-// 256^3 FP32 24 / 32 / 43 / 64 / 128 planes 279 / 274 / 283 / 327 / 379;
-// 512^3 FP16 64 / 256 planes 1,745 / 2,519; 128^3 FP32 13 / 16 / 20 / 32
-// planes 41.5 / 45.2 / 47.4 / 61.7.
+// Whether the D3Q19 bulk sets run with three CTAs an SM (F_DENSE): domains with
+// 24 planes of columns or more for each of those CTAs' places.
+static bool dense_domain(const mrlbm_domain* dom)
+{
+    const mrlbm_desc& d = dom->d;
+    const long long cols = (long long)((d.nx + TILE_X - 1) / TILE_X) * ((d.ny + TYI_BULK - 1) / TYI_BULK);
+    return cols * d.nz >= 24LL * dom->nsm * step_ctas(19, F_DENSE, TYI_BULK);
+}
+
+// Whether the D3Q27 bulk sets run in the sums march: always with FP32 moments.
+// 16-bit ones cost it a conversion of each of the rows it reads, so it gains
+// only where many tiles hide its longer steps (256^3 FP16 2,501 us per 10
+// steps against 2,827; 100 x 90 x 80, 20 steps, 456 against 442 at the same
+// chunk, 743 against 549 alone).  The line is drawn at the cross-section, 256
+// columns, so that the slabs of a domain cut in z run the kernel of the whole.
+static bool sums_domain(const mrlbm_domain* dom)
+{
+    const mrlbm_desc& d = dom->d;
+    return d.storage == MRLBM_F32 ||
+           (long long)((d.nx + TILE_X - 1) / TILE_X) * ((d.ny + TYI_BULK - 1) / TYI_BULK) >= 256;
+}
+
+// z planes per CTA of the sums march: even chunks of at most 32 planes (48 with
+// 16-bit moments: 256^3 FP16 32 / 43 / 64 planes 262 / 250 / 248 us a step)
+// that make 1.4 waves of CTAs; a domain that has not as many at 8 planes takes the
+// shortest chunk that fits one wave.  Longer chunks save their two lead planes
+// (6 % at 32), but neighbouring columns then drift apart and re-read their
+// halo rows from DRAM instead of L2, and a step of few tiles waits for whole
+// columns.  Measured (us a step, alone): 256^3 FP32 24 / 32 / 43 / 64 / 128
+// planes 279 / 274 / 283 / 327 / 379; 512^3 FP16 64 / 256 planes 1,745 /
+// 2,519; 128^3 FP32 13 / 16 / 20 / 32 planes 41.5 / 45.2 / 47.4 / 61.7; 64^3
+// 3 / 4 / 8 planes 11.7 / 13.6 / 18.9 (among others 7.6 / 6.7 / 7.1; the 27
+// populations at 4 planes 12.5 and 8.9).
 int mrlbm::choose_lz_sums(const mrlbm_domain* dom)
 {
     const mrlbm_desc& d = dom->d;
     const long long cols = (long long)((d.nx + TILE_X - 1) / TILE_X) * ((d.ny + TYI_BULK - 1) / TYI_BULK);
     const long long slots = (long long)dom->nsm * SUM_CTAS;
-    int lz = std::min(d.nz, 32);
-    while (lz > 8 && 5 * cols * ((d.nz + lz - 1) / lz) < 7 * slots) lz--;
+    auto ctas = [&](int lz) { return cols * ((d.nz + lz - 1) / lz); };
+    const int most = d.storage == MRLBM_F32 ? 32 : 48, nzc = (d.nz + most - 1) / most;
+    int lz = (d.nz + nzc - 1) / nzc;
+    while (lz > 8 && 5 * ctas(lz) < 7 * slots) lz--;
+    if (5 * ctas(lz) < 7 * slots && lz <= 8) {
+        const int top = lz;
+        lz = std::min(2, top);
+        while (lz < top && ctas(lz) > slots) lz++;
+    }
     return lz;
 }
 
@@ -581,15 +621,10 @@ mrlbm_status mrlbm::classify_nodes(int q, int mq, const uint32_t* nt, long long 
     // whether a node takes the total sums depends on its mask and on which of
     // the x and y faces it lies on only: -1 not worked out yet
     std::vector<int8_t> totals_of(geom ? 256 * 16 : 0, (int8_t)-1);
-    int x = -1, y = 0;
     table.assign(1, BcClass{});  // class 0: bulk (unused entry)
     cls.resize(n);
     any_bc = false;
     for (long long k = 0; k < n; k++) {
-        if (geom && ++x == geom->nx) {
-            x = 0;
-            if (++y == geom->ny) y = 0;
-        }
         const uint32_t w = nt[k];
         // run-time classes key on the octant mask, BC kind and velocity index;
         // case mode hands the whole word to the case's own snippet (like the
@@ -603,6 +638,8 @@ mrlbm_status mrlbm::classify_nodes(int q, int mq, const uint32_t* nt, long long 
         const uint32_t key = case_mode ? w : (w & key_bits);
         bool totals = false;
         if (geom && ((w >> 8) & 7u) != 2u) {
+            const uint64_t row = (uint64_t)k / (uint32_t)geom->nx;
+            const int x = (int)((uint64_t)k - row * (uint32_t)geom->nx), y = (int)(row % (uint32_t)geom->ny);
             const int face = (x == 0) | (x == geom->nx - 1) << 1 | (y == 0) << 2 | (y == geom->ny - 1) << 3;
             int8_t& t = totals_of[(w & 0xFFu) * 16 + face];
             if (t < 0) t = takes_totals(*geom, q, known_mask(q, w & 0xFFu), x, y);
@@ -834,9 +871,12 @@ void mrlbm::fill_step_args(const mrlbm_domain* dom, StepArgs& a, int parity, int
     if (d.thermal) flags |= F_THERMAL | F_FORCE;           // the Boussinesq force is per node
     if (dom->has_outflow) flags |= F_OUTFLOW;
     if (d.storage == MRLBM_F16U) flags |= F_SPLITU;
+    if (dom->q == 19 && dom->dense && (flags & ~F_FORCE) == 0) flags |= F_DENSE;
+    if (dom->q == 27 && dom->sums && (flags & ~(F_FORCE | F_SPLITU)) == 0) flags |= F_SUMS;
     const int kind = tile_kind(tile_rows(flags));
     a.lz = dom->lz > 0                 ? dom->lz
            : sums_march(dom->q, flags) ? dom->lz_s
+           : (flags & F_DENSE)         ? dom->lz_b[tile_ordered(dom, flags) ? 1 : 0]
            : tile_ordered(dom, flags)  ? dom->lz_o[kind]
                                        : dom->lz_t[kind];
 }

@@ -46,10 +46,13 @@ static mrlbm_status launch_step_t(const CUtensorMap* maps, const StepArgs& a, cu
 template <int Q, typename T>
 mrlbm_status dispatch_step(const CUtensorMap* maps, const StepArgs& a, int flags, cudaStream_t s, bool pdl)
 {
+    // (the FP32 D3Q27 bulk sets all run the sums march)
+    if constexpr (!(Q == 27 && is_f32<T>())) {
+        if (flags == 0) return launch_step_t<Q, T, 0>(maps, a, s, pdl);
+        if (flags == F_FORCE) return launch_step_t<Q, T, F_FORCE>(maps, a, s, pdl);
+    }
     switch (flags) {
-        case 0: return launch_step_t<Q, T, 0>(maps, a, s, pdl);
         case F_BC: return launch_step_t<Q, T, F_BC>(maps, a, s, pdl);
-        case F_FORCE: return launch_step_t<Q, T, F_FORCE>(maps, a, s, pdl);
         case F_BC | F_FORCE: return launch_step_t<Q, T, F_BC | F_FORCE>(maps, a, s, pdl);
         case F_BC | F_POWERLAW: return launch_step_t<Q, T, F_BC | F_POWERLAW>(maps, a, s, pdl);
         case F_BC | F_FORCE | F_POWERLAW: return launch_step_t<Q, T, F_BC | F_FORCE | F_POWERLAW>(maps, a, s, pdl);
@@ -59,6 +62,18 @@ mrlbm_status dispatch_step(const CUtensorMap* maps, const StepArgs& a, int flags
         case F_BC | F_OUTFLOW: return launch_step_t<Q, T, F_BC, OutflowBC>(maps, a, s, pdl);
         case F_BC | F_FORCE | F_OUTFLOW: return launch_step_t<Q, T, F_BC | F_FORCE, OutflowBC>(maps, a, s, pdl);
         default: break;
+    }
+    if constexpr (Q == 19) {
+        if (flags == F_DENSE) return launch_step_t<Q, T, F_DENSE>(maps, a, s, pdl);
+        if (flags == (F_DENSE | F_FORCE)) return launch_step_t<Q, T, F_DENSE | F_FORCE>(maps, a, s, pdl);
+    } else {
+        if (flags == F_SUMS) return launch_step_t<Q, T, F_SUMS>(maps, a, s, pdl);
+        if (flags == (F_SUMS | F_FORCE)) return launch_step_t<Q, T, F_SUMS | F_FORCE>(maps, a, s, pdl);
+        if constexpr (std::is_same<T, __half>::value) {
+            if (flags == (F_SUMS | F_SPLITU)) return launch_step_t<Q, T, F_SUMS | F_SPLITU>(maps, a, s, pdl);
+            if (flags == (F_SUMS | F_SPLITU | F_FORCE))
+                return launch_step_t<Q, T, F_SUMS | F_SPLITU | F_FORCE>(maps, a, s, pdl);
+        }
     }
     // split-velocity 16-bit storage (no thermal scalar, no outflow walls)
     if constexpr (std::is_same<T, __half>::value) {

@@ -21,7 +21,8 @@
 // populations (one row a lane, packed shared-memory row exchange); 252 thread
 // instructions a node against 379; DRAM traffic 1.076 times the algorithmic
 // bytes; 512^3 FP16 1,820 us against 2,117.  What bounds it: 5.0 TB/s of the
-// 6.5 TB/s copy rate, with 13 warps an SM at 57 % issue.  R = 1 (one row a
+// 6.5 TB/s copy rate, with 13 warps an SM at 45 % issue.  Which domains run it:
+// sums_domain.  R = 1 (one row a
 // lane, 27 warps) took 313 us: 339 instructions, and the many columns in
 // flight re-read their halos from DRAM (1.21 times).
 //

@@ -18,6 +18,7 @@ import parity_util as pu
 pytestmark = pytest.mark.gpu
 EPS = 6e-8
 STEPS = 6
+WALL_LOW, WALL_SECOND = 2e-5, 3e-4   # whole populations: eps / u^2 on the second moments, as in test_gpu_parity
 SHAPES = [(31, 7, 1), (32, 8, 3), (33, 9, 2), (1, 12, 10), (12, 1, 5), (9, 5, 1), (64, 16, 33), (65, 17, 40), (2, 2, 2),
           (40, 23, 67)]
 
@@ -56,8 +57,10 @@ def test_d3q27_bulk(shape, force):
 
 
 @pytest.mark.parametrize("storage,ulp", [(mrlbm.F16, 2.0 ** -11), (mrlbm.BF16, 2.0 ** -8), (mrlbm.F16U, 2.0 ** -20)])
-@pytest.mark.parametrize("shape", [(33, 9, 2), (64, 16, 33)])
+@pytest.mark.parametrize("shape", [(33, 9, 2), (512, 120, 2), (512, 128, 2), (515, 130, 3)])
 def test_d3q27_16bit(shape, storage, ulp):
+    """Both sides of the cross-section from which 16-bit moments take the sums
+    march (256 columns of 32 x 8 nodes)."""
     d = mrlbm.make_desc(*shape, lattice=mrlbm.D3Q27, storage=storage, tau=0.6)
     low, second = errors(d)
     # split storage keeps the second moments (and the little they give u) in one fp16 word
@@ -65,9 +68,28 @@ def test_d3q27_16bit(shape, storage, ulp):
     assert second < 4 * STEPS * max(ulp, 2.0 ** -11), second
 
 
+@pytest.mark.parametrize("nz", [2660, 2700])   # 4 columns: under and over 24 planes a CTA's place (10,656)
+def test_d3q19_dense(nz):
+    """The three-CTA shape of the D3Q19 bulk step, against the oracle, and bit
+    for bit against the batch kernel (which has one shape)."""
+    nx, ny = 33, 9
+    d = mrlbm.make_desc(nx, ny, nz, lattice=mrlbm.D3Q19, tau=0.56)
+    low, second = errors(d)
+    assert low < WALL_LOW and second < WALL_SECOND, (low, second)
+    dom, b = mrlbm.Domain(d), mrlbm.Batch(mrlbm.D3Q19, mrlbm.F32)
+    m = b.add(d)
+    f = flow((nz, ny, nx), 5)
+    dom.init_flow(*f)
+    m.init_flow(*f)
+    dom.step(STEPS)
+    b.step(STEPS)
+    assert np.array_equal(dom.moments(), m.moments())
+    b.close()
+    dom.close()
+
+
 # ---- walls that take the total sums (x and y faces) and the class table's order
 
-WALL_LOW, WALL_SECOND = 2e-5, 3e-4   # whole populations: eps / u^2 on the second moments, as in test_gpu_parity
 
 
 def wall_errors(d, nt):
