@@ -1806,8 +1806,9 @@ __device__ __forceinline__ bool zmarch_column(const StepArgs& a, const CUtensorM
 namespace mrlbm {
 
 // Barriers, the timeout flag and, in wall kernels, the staged copy of the
-// first ZSmem::CT classes of the table bc (nbc classes)
-template <typename SMT>
+// first ZSmem::CT classes of the table bc (nbc classes).  SYNC: ends with a CTA
+// barrier; without, the caller's next one makes it visible.
+template <bool SYNC = true, typename SMT>
 __device__ __forceinline__ void zmarch_init_barriers(const SMT& sm, const BcClass* bc = nullptr, int nbc = 0)
 {
     int staged = 0;
@@ -1824,7 +1825,7 @@ __device__ __forceinline__ void zmarch_init_barriers(const SMT& sm, const BcClas
         for (int s = 0; s < SMT::NS; s++) mbar_init(&sm.bars[s], 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    __syncthreads();
+    if (SYNC) __syncthreads();
 }
 
 // Tile-ordered steps.  Each launch of the single-domain step may begin while
@@ -1854,14 +1855,18 @@ __device__ __forceinline__ unsigned ld_acquire_u32(const unsigned* p)
 }
 
 // Takes the CTA's ticket and waits for the tiles around its tile; returns the
-// step index and sets the tile.  Ends with no CTA barrier: the caller's next
-// one orders the waits before the tile's first load.
-__device__ __forceinline__ unsigned tile_order_begin(const StepArgs& a, int& tx, int& ty, int& kc)
+// step index and sets the tile.  meanwhile: work of the CTA that needs neither
+// (its set-up), done while the ticket is on its way.  Ends with no CTA barrier:
+// the caller's next one orders the waits before the tile's first load.
+template <typename F>
+__device__ __forceinline__ unsigned tile_order_begin(const StepArgs& a, int& tx, int& ty, int& kc, F&& meanwhile)
 {
     unsigned* hdr = reinterpret_cast<unsigned*>(dyn_smem() + HDR_TICKET);
     const unsigned ncol = gridDim.x * gridDim.y, ntile = ncol * gridDim.z;
+    unsigned long long t = 0;
+    if (threadIdx.x == 0) t = atomicAdd(reinterpret_cast<unsigned long long*>(a.sched), 1ull);
+    meanwhile();
     if (threadIdx.x == 0) {
-        const unsigned long long t = atomicAdd(reinterpret_cast<unsigned long long*>(a.sched), 1ull);
         hdr[0] = (unsigned)(t % ntile);
         hdr[1] = (unsigned)(t / ntile);
     }
@@ -1942,8 +1947,17 @@ __global__ void __launch_bounds__(32 * step_warps(Q, FLAGS, TYI), step_ctas(Q, F
     const step_smem_t<Q, T, FLAGS, TYI, BCP> sm(smem);
     int tx = blockIdx.x, ty = blockIdx.y, kc = blockIdx.z;
     unsigned s = 0;
-    if (a.sched) s = tile_order_begin(a, tx, ty, kc);
-    zmarch_init_barriers(sm, a.bc, a.nbc);  // ends with a CTA barrier
+    // A short chunk's CTA lives a few us, a good part of it before its first
+    // plane lands: the tensor map is fetched and the set-up done while the
+    // ticket is on its way (64^3 cavity per 50 steps 455 us against 470
+    // among others, 615 against 655 alone).
+    if (threadIdx.x == 32) asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&map_in)) : "memory");
+    if (a.sched) {
+        s = tile_order_begin(a, tx, ty, kc, [&] { zmarch_init_barriers<false>(sm, a.bc, a.nbc); });
+    } else {
+        zmarch_init_barriers<false>(sm, a.bc, a.nbc);
+    }
+    __syncthreads();
     // the tiles' stores of the previous step were made visible to this
     // thread through the generic proxy; the ring's loads use the async one
     if (a.sched) asm volatile("fence.proxy.async.global;" ::: "memory");
