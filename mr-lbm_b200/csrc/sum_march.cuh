@@ -308,7 +308,8 @@ __device__ __forceinline__ void edge_into(float (&q)[6], const float* e, bool on
         "@p ld.shared.v4.f32 {%0, %1, %2, %3}, [%6];\n\t"
         "@p ld.shared.v2.f32 {%4, %5}, [%6 + 16];\n\t}"
         : "+f"(q[0]), "+f"(q[1]), "+f"(q[2]), "+f"(q[3]), "+f"(q[4]), "+f"(q[5])
-        : "r"((unsigned)__cvta_generic_to_shared(e)), "r"((int)on));
+        : "r"((unsigned)__cvta_generic_to_shared(e)), "r"((int)on)
+        : "memory");
 }
 __device__ __forceinline__ void edge_into(F2 (&q)[6], const float* e, bool on)
 {
@@ -322,7 +323,8 @@ __device__ __forceinline__ void edge_into(F2 (&q)[6], const float* e, bool on)
         "@p ld.shared.v2.b64 {%2, %3}, [%6 + 16];\n\t"
         "@p ld.shared.v2.b64 {%4, %5}, [%6 + 32];\n\t}"
         : "+l"(q[0].v), "+l"(q[1].v), "+l"(q[2].v), "+l"(q[3].v), "+l"(q[4].v), "+l"(q[5].v)
-        : "r"((unsigned)__cvta_generic_to_shared(e)), "r"((int)on));
+        : "r"((unsigned)__cvta_generic_to_shared(e)), "r"((int)on)
+        : "memory");
 }
 
 __device__ __forceinline__ float from_left(float v) { return __shfl_up_sync(0xffffffffu, v, 1); }
