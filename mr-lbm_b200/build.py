@@ -8,7 +8,8 @@ exchange buffers; for tests only).
 Every translation unit under csrc/ is compiled by nvcc for
 `-gencode arch=compute_100a,code=sm_100a` in parallel into _build/ (and
 _build_check/), then linked.  Objects are rebuilt when any source or header
-under csrc/ (or include/) is newer than the object.
+under csrc/ (or include/) is newer than the object.  ptxas's lines on each
+kernel (registers, spilled bytes) are kept beside the object (.ptxas).
 """
 import argparse
 import concurrent.futures as cf
@@ -27,11 +28,15 @@ BUILD, LIB, _ = VARIANTS[""]
 NVCC = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 FLAGS = ["-O3", "-lineinfo", "-std=c++17", "--expt-relaxed-constexpr", "-Xcompiler", "-fPIC",
-         "-ccbin", "/usr/bin/g++", "-I", os.path.join(ROOT, "include")]
+         "-ccbin", "/usr/bin/g++", "-I", os.path.join(ROOT, "include"), "-Xptxas", "-v"]
 
 
 def _newest(paths):
     return max(os.path.getmtime(p) for p in paths) if paths else 0.0
+
+
+def _ptxas(obj):
+    return obj[:-2] + ".ptxas"
 
 
 def build(force=False, jobs=None, verbose=False, extra_flags=(), check=True):
@@ -55,7 +60,8 @@ def build_variant(name, force=False, jobs=None, verbose=False, extra_flags=()):
     for src in sources:
         obj = os.path.join(BUILD, os.path.basename(src)[:-3] + ".o")
         objs.append(obj)
-        if force or not os.path.exists(obj) or os.path.getmtime(obj) < max(os.path.getmtime(src), hdr_time):
+        if force or not all(map(os.path.exists, (obj, _ptxas(obj)))) or \
+                os.path.getmtime(obj) < max(os.path.getmtime(src), hdr_time):
             todo.append((src, obj))
 
     def compile_one(item):
@@ -64,7 +70,9 @@ def build_variant(name, force=False, jobs=None, verbose=False, extra_flags=()):
         r = subprocess.run(cmd, capture_output=True, text=True)
         if r.returncode != 0:
             raise RuntimeError("nvcc failed for %s:\n%s\n%s" % (src, r.stdout, r.stderr))
-        return src, r.stderr
+        with open(_ptxas(obj), "w") as f:
+            f.write(r.stderr)
+        return src, "".join(s for s in r.stderr.splitlines(True) if "ptxas info" not in s and "bytes stack frame" not in s)
 
     if todo:
         n = jobs or min(len(todo), os.cpu_count() or 4)

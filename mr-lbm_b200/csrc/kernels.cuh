@@ -462,10 +462,13 @@ __device__ __forceinline__ void class_row(const float* w, float (&r)[8])
 // 16-byte loads; in kernels of many sets, or next to another inlined copy of
 // the solve, they spill, so those read a word at a time.  TOT: classes marked
 // BC_TOTALS take the total sums, rho (1, Pi_hat) of the bulk moments that mac
-// holds on entry (the kernels without a staged table; in the others the second
-// way to the sums costs spills: 128^3 D3Q19 cavity +13 %).  XC: the rows' last
+// holds on entry: the kernels whose domains have such classes, D3Q27 and
+// thermal ones (a D3Q19 outflow channel of 180 x 160 x 150 took 149 us a step
+// against 139 with the branch in, and spilled; in the kernels with a staged
+// table it costs spills too: 128^3 D3Q19 cavity +13 %).  XC: the rows' last
 // word is read where no class takes totals either, as the zero it then is (in
-// the kernels with two solves inlined ptxas spills 12 bytes with it, 44 without).
+// the staged copy's solve of TableBCShared ptxas spills 16 bytes with it, 48
+// without).
 template <int Q, bool SH = false, bool VEC = false, bool TOT = false, bool XC = TOT>
 __device__ __forceinline__ void bc_moments(const BcClass* __restrict__ c, const float* p, float omega,
                                            float omega0, float* mac)
@@ -605,7 +608,7 @@ struct OutflowBC {
         const BcClass* c = a.bc + cls;
         const uint32_t kw = __ldg(&c->trule);
         if (((kw >> 8) & 7u) == BC_KIND_OUTFLOW) outflow_moments<T>(a, kw, x, y, z, mac);
-        else bc_moments<Q, false, false, true>(c, p, omega, a.omega0, mac);
+        else bc_moments<Q, false, false, Q == 27>(c, p, omega, a.omega0, mac);   // no D3Q19 class takes totals here
     }
     template <typename T>
     static __device__ __forceinline__ void thermal(const StepArgs& a, uint8_t cls, const float* pg, unsigned oidx,
@@ -625,7 +628,7 @@ struct TableBCShared : TableBC {
                                                  int x, int y, int z, float* mac)
     {
         if ((int)cls < staged_classes()) bc_moments<Q, true, false, false, true>(staged_class(cls), p, omega, a.omega0, mac);
-        else bc_moments<Q, false, false, false, true>(a.bc + cls, p, omega, a.omega0, mac);
+        else bc_moments<Q>(a.bc + cls, p, omega, a.omega0, mac);
     }
 };
 

@@ -1,0 +1,38 @@
+"""What ptxas reports of the step kernels (the .ptxas files that build.py keeps
+beside the objects): which of them spill registers, and how much."""
+import glob
+import os
+import re
+
+import pytest
+
+HERE = os.path.dirname(os.path.abspath(__file__))
+LOGS = os.path.join(os.path.dirname(HERE), "mr-lbm_b200", "_build", "step_*.ptxas")
+
+
+def spilled():
+    """Bytes of spill stores and loads by kernel (mangled name)."""
+    out = {}
+    for path in glob.glob(LOGS):
+        name = None
+        with open(path) as f:
+            for line in f:
+                m = re.search(r"Compiling entry function '(\S+)'", line)
+                name = m.group(1) if m else name
+                m = re.search(r"(\d+) bytes spill stores, (\d+) bytes spill loads", line)
+                if m and name:
+                    out[name] = int(m.group(1)) + int(m.group(2))
+    if not out:
+        pytest.skip("the library was not built here")
+    return out
+
+
+def test_d3q19_outflow_kernels_do_not_spill():
+    """96 registers hold them; a branch that no D3Q19 class takes once cost 5-10 %."""
+    s = {k: v for k, v in spilled().items() if "OutflowBC" in k and "Li19E" in k}
+    assert len(s) == 6 and not any(s.values()), s
+
+
+def test_no_step_kernel_spills_much():
+    """A dozen words at most, none of them in the loads of a plane."""
+    assert max(spilled().values()) <= 48, {k: v for k, v in spilled().items() if v > 48}
