@@ -1511,6 +1511,10 @@ struct ZRing {
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
             for (int s = 0; s < NS && s < nprod; s++) load_slot(slot(s), s);
         }
+        // The warp's other lanes go on to wait for these loads: not before
+        // their own lane has issued them, which their polling could hold up.
+        // (Later loads are issued a CTA barrier ahead of any wait for them.)
+        __syncwarp();
     }
     // CTA-wide timeout flag next to the ring barriers: a thread whose bounded
     // wait gave up raises it before the per-plane barrier, every thread reads

@@ -108,3 +108,27 @@ def test_large_grid_matches_and_reports_no_timeout():
     ref = run(d, 40, 0, order=False, tgv=tg)
     got = run(d, 40, 0, order=True, tgv=tg)
     same(got, ref)
+
+
+@pytest.mark.parametrize("q,walls", [(19, True), (27, False), (27, True)])
+def test_many_short_steps(q, walls):
+    """Some 10^7 first loads, each awaited by the lanes of the warp whose own
+    lane issues them: no wait runs out (synchronize raises), and the steps in
+    flight at a time do not change the result."""
+    if walls:
+        d, nt = mrlbm.lid_cavity_desc(32, re=100.0, lid_u=0.05, lattice=q), mrlbm.lid_cavity_node_types(32, 32, 32, 1)
+    else:
+        d, nt = mrlbm.make_desc(32, 32, 32, lattice=q, tau=0.8), None
+    doms = [mrlbm.Domain(d) for _ in range(2)]
+    for dom in doms:
+        if nt is not None:
+            dom.set_node_types(nt)
+        dom.init_uniform((0.01, 0.005, 0.002))
+    doms[0].step(30000)
+    for _ in range(30):
+        doms[1].step(1000)
+    for dom in doms:
+        dom.synchronize()
+    same(*(dom.moments() for dom in doms))
+    for dom in doms:
+        dom.close()
