@@ -118,7 +118,7 @@ __host__ __device__ constexpr int tile_kind(int tyi) { return tyi == TYI_BULK ? 
 __host__ __device__ constexpr int tile_rows_of_kind(int kind) { return kind == 0 ? TYI_BULK : TYI_WALL; }
 constexpr uint8_t CLS_BULK = 0;
 constexpr uint8_t CLS_SOLID = 255;
-constexpr unsigned WAIT_LIMIT = 1u << 26;  // mbarrier polls before giving up (~seconds)
+constexpr unsigned WAIT_LIMIT = 1u << 20;  // mbarrier polls before giving up (4 us each: 4 s)
 constexpr unsigned DEP_LIMIT = 1u << 21;   // tile-order polls (an L2 round trip + 64 ns each, ~seconds)
 
 // Bounds-check build (-DMRLBM_BOUNDS_CHECK, libmrlbm_check.so): every

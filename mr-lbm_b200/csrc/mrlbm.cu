@@ -1073,7 +1073,8 @@ __global__ void bounded_wait_selftest_kernel(int* err, unsigned polls)
 
 extern "C" mrlbm_status mrlbm_selftest_bounded_wait(unsigned polls, double* seconds)
 {
-    if (polls == 0 || polls > WAIT_LIMIT) return fail(MRLBM_EINVAL, "polls must be in 1..%u", WAIT_LIMIT);
+    constexpr unsigned most = 1u << 26;
+    if (polls == 0 || polls > most) return fail(MRLBM_EINVAL, "polls must be in 1..%u", most);
     int* d_err = nullptr;
     CK(cudaMalloc(&d_err, sizeof(int)));
     cudaError_t e = cudaMemset(d_err, 0, sizeof(int));

@@ -7,6 +7,9 @@ chunks), tile grids of one tile along an axis, periodic and walled axes,
 16-bit storage, and mixes with graph replay and with a z chunk changed
 between calls.
 """
+import os
+import re
+
 import numpy as np
 import pytest
 
@@ -132,3 +135,15 @@ def test_many_short_steps(q, walls):
     same(*(dom.moments() for dom in doms))
     for dom in doms:
         dom.close()
+
+
+def test_the_step_kernels_waits_last_seconds():
+    """The limit of the tile waits in seconds, from its polls and the time of
+    a poll: long against any load, short against a hung device (a limit of
+    2^26 once held a step for 266 s)."""
+    here = os.path.dirname(os.path.abspath(__file__))
+    with open(os.path.join(os.path.dirname(here), "mr-lbm_b200", "csrc", "kernels.cuh")) as f:
+        limit = 1 << int(re.search(r"WAIT_LIMIT = 1u << (\d+)", f.read()).group(1))
+    st, sec = mrlbm.selftest_bounded_wait(1 << 15)
+    assert st == 6
+    assert 0.5 < sec / (1 << 15) * limit < 20.0
