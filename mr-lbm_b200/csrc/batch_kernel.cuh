@@ -65,7 +65,7 @@ __device__ __forceinline__ bool batch_column(
         return sum_column<T, FLAGS, TYI, 1>(a, map, it.X0, it.Y0, it.z0, min(it.z0 + a.lz, a.nz), sm, g0);
     // one generic-pointer solve for every flag set: the batch kernel holds
     // them all, and two inlined solves per set spill
-    using BCP = std::conditional_t<batch_stages(Q), TableBCGeneric<false>, TableBC>;
+    using BCP = std::conditional_t<batch_stages(Q), TableBCGeneric<false>, table_policy_t<Q, FLAGS>>;
     return zmarch_column<Q, T, FLAGS, TYI, BCP>(a, map, it.X0, it.Y0, it.z0, min(it.z0 + a.lz, a.nz), sm, g0);
 }
 

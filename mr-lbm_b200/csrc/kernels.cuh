@@ -466,9 +466,10 @@ __device__ __forceinline__ void class_row(const float* w, float (&r)[8])
 // thermal ones (a D3Q19 outflow channel of 180 x 160 x 150 took 149 us a step
 // against 139 with the branch in, and spilled; in the kernels with a staged
 // table it costs spills too: 128^3 D3Q19 cavity +13 %).  XC: the rows' last
-// word is read where no class takes totals either, as the zero it then is (in
-// the staged copy's solve of TableBCShared ptxas spills 16 bytes with it, 48
-// without).
+// word, the totals' constant, is read in every class as the zero it is in the
+// others: the totals solve is 1-2 % faster so on a cavity, and in the staged
+// copy's solve of TableBCShared, where no class takes totals, ptxas spills 16
+// bytes with it and 48 without.
 template <int Q, bool SH = false, bool VEC = false, bool TOT = false, bool XC = TOT>
 __device__ __forceinline__ void bc_moments(const BcClass* __restrict__ c, const float* p, float omega,
                                            float omega0, float* mac)
@@ -491,6 +492,7 @@ __device__ __forceinline__ void bc_moments(const BcClass* __restrict__ c, const 
             for (int k = 0; k < (XC ? 8 : 7); k++) w[k] = class_word<SH>(&c->ainv[r][k]);
         }
         float acc = XC ? w[7] : 0.f;   // 0 in classes that take no totals
+        if (TOT && !XC && (known & BC_TOTALS)) acc = class_word<SH>(&c->ainv[r][7]);
 #pragma unroll
         for (int k = 0; k < 7; k++) acc = fmaf(w[k], b[k], acc);
         X[r] = acc;
@@ -583,13 +585,20 @@ __device__ __forceinline__ const BcClass* staged_class(int cls)
 }
 // The run-time class table, read from global memory (D3Q27, thermal and
 // batch kernels: a second inlined copy of the solve, or the shared copy's
-// generic loads, measured slower or spilled there).
-struct TableBC {
+// generic loads, measured slower or spilled there).  XC (bc_moments): off in
+// the D3Q27 sets with a force or a non-Newtonian viscosity, which are the
+// ducts and porous boxes whose lanes hold many classes, few of them with
+// totals.  96^3 duct with 5 % scattered obstacles, us a step with the word
+// read only in totals classes / in all / without totals: FP32 Newtonian
+// 67.9 / 75.3 / 73.3, power law 90.5 / 97.5 / 94.2, Bingham 88.0 / 96.1 / 90.7;
+// 128^3 cavity 71.9 / 70.6 / 75.0.
+template <bool XC>
+struct TableBCRows {
     template <int Q, typename T>
     static __device__ __forceinline__ void apply(const StepArgs& a, uint8_t cls, const float* p, float omega,
                                                  int x, int y, int z, float* mac)
     {
-        bc_moments<Q, false, false, true>(a.bc + cls, p, omega, a.omega0, mac);
+        bc_moments<Q, false, false, true, XC>(a.bc + cls, p, omega, a.omega0, mac);
     }
     // C and 3 sum g c at a thermal boundary node: the class's run-time rule
     template <typename T>
@@ -599,6 +608,7 @@ struct TableBC {
         thermal_wall(a, a.bc + cls, pg, oidx, C, q);
     }
 };
+using TableBC = TableBCRows<true>;
 
 struct OutflowBC {
     template <int Q, typename T>
@@ -664,7 +674,7 @@ template <int Q, int FLAGS>
 using table_policy_t =
     std::conditional_t<Q == 19 && (FLAGS & F_THERMAL) == 0,
                        std::conditional_t<(FLAGS & (F_POWERLAW | F_BINGHAM)) != 0, TableBCGeneric<true>, TableBCShared>,
-                       TableBC>;
+                       TableBCRows<(FLAGS & F_THERMAL) != 0 || (FLAGS & (F_FORCE | F_POWERLAW | F_BINGHAM)) == 0>>;
 
 // Power-law omega by Newton iteration (src/nnf.h:61-89 with its compile
 // defects fixed) and Bingham (src/nnf.h:92-98).
