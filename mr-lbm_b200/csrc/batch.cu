@@ -114,14 +114,20 @@ int batch_flags(const mrlbm_domain* dom)
     int flags;
     fill_step_args(dom, a, 0, flags);
     flags &= ~F_DENSE;   // a launch shape of the single-domain step
-    if (flags & (F_FORCE | F_POWERLAW | F_BINGHAM)) flags = (flags & ~F_SUMS) | F_BC;
+    // forced members run the walls' kernel, but those of the sums march stay in it (as alone)
+    if (!(flags & F_SUMS) && (flags & (F_FORCE | F_POWERLAW | F_BINGHAM))) flags |= F_BC;
     return flags;
 }
 
-bool flags_supported(int f)
+// the sets that batch_step's switch has a body for
+bool flags_supported(const mrlbm_batch* b, int f)
 {
-    f &= ~(F_SPLITU | F_SUMS);  // every set below also with split-velocity storage, or in the sums march
-    return f == 0 || f == F_BC || f == (F_BC | F_FORCE) || f == (F_BC | F_FORCE | F_POWERLAW);
+    const int split = b->storage == MRLBM_F16U ? F_SPLITU : 0;
+    if ((f & F_SPLITU) != split) return false;
+    f &= ~F_SPLITU;
+    if (f == F_SUMS || f == (F_SUMS | F_FORCE)) return b->lattice == 27;
+    if (f == 0) return !(b->lattice == 27 && b->storage == MRLBM_F32);
+    return f == F_BC || f == (F_BC | F_FORCE) || f == (F_BC | F_FORCE | F_POWERLAW);
 }
 
 // Rebuild the per-domain records and the work list from the members; upload
@@ -149,7 +155,7 @@ mrlbm_status refresh(mrlbm_batch* b)
         int f;
         for (int p = 0; p < 2; p++) fill_step_args(dom, hd[id].args[p], p, f);
         hd[id].flags = batch_flags(dom);
-        if (!flags_supported(hd[id].flags))
+        if (!flags_supported(b, hd[id].flags))
             return fail(MRLBM_EINVAL, "batch member %d: physics flag set %d not supported in batches", id, hd[id].flags);
         if (dom->has_outflow)
             return fail(MRLBM_EINVAL, "batch member %d: outflow walls are not supported in batches", id);
@@ -299,7 +305,7 @@ extern "C" mrlbm_status mrlbm_batch_add(mrlbm_batch* b, const mrlbm_desc* desc, 
     mrlbm_domain* dom = nullptr;
     mrlbm_status st = mrlbm_domain_create(desc, &dom);
     if (st) return st;
-    if (!flags_supported(batch_flags(dom))) {
+    if (!flags_supported(b, batch_flags(dom))) {
         mrlbm_domain_destroy(dom);
         return fail(MRLBM_EINVAL, "physics of this domain are not supported in batches");
     }

@@ -115,12 +115,16 @@ __global__ void __launch_bounds__(32 * (TYI + 2), ctas_per_sm(TYI))
         __syncthreads();
         bool ok = true;
         switch (D.flags) {
-            // (FP32 D3Q27 members without walls are all in the sums march)
+            // (the sets with a body here: flags_supported; FP32 D3Q27 members
+            // without walls are all in the sums march)
             case S:
                 if constexpr (!(Q == 27 && is_f32<T>())) ok = batch_column<Q, T, S, TYI>(s_args, &D.map[par], item, sm, g0);
                 break;
             case S | F_SUMS:
                 if constexpr (Q == 27) ok = batch_column<Q, T, S | F_SUMS, TYI>(s_args, &D.map[par], item, sm, g0);
+                break;
+            case S | F_SUMS | F_FORCE:
+                if constexpr (Q == 27) ok = batch_column<Q, T, S | F_SUMS | F_FORCE, TYI>(s_args, &D.map[par], item, sm, g0);
                 break;
             case S | F_BC: ok = batch_column<Q, T, S | F_BC, TYI>(s_args, &D.map[par], item, sm, g0); break;
             case S | F_BC | F_FORCE: ok = batch_column<Q, T, S | F_BC | F_FORCE, TYI>(s_args, &D.map[par], item, sm, g0); break;

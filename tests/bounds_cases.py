@@ -78,6 +78,28 @@ def cases():
         return _run(d, nt, lambda dom: dom.init_uniform())
     out["thermal_plates"] = thermal
 
+    def batch27(rows):
+        # the sums march and the walls, chained in the same CTAs
+        b = mrlbm.Batch(mrlbm.D3Q27, mrlbm.F32)
+        b.set_rows(rows)
+        mem = []
+        for nx, ny, nz, force in ((33, 15, 7, 0.0), (20, 20, 9, 1e-5), (64, 14, 33, 0.0)):
+            mem.append(b.add(mrlbm.make_desc(nx, ny, nz, lattice=27, tau=0.7, force=(force, 0.0, 0.0))))
+            mem[-1].init_flow(*_flow((nz, ny, nx), nx + ny + nz))
+        for nx, ny, nz in ((33, 15, 7), (20, 9, 5)):
+            mem.append(b.add(mrlbm.lid_cavity_desc(nx, re=100.0, lid_u=0.05, lattice=27, ny=ny, nz=nz)))
+            mem[-1].set_node_types(mrlbm.lid_cavity_node_types(nx, ny, nz, 1))
+            mem[-1].init_uniform()
+        b.step(STEPS)
+        b.synchronize()
+        for m in mem:
+            m.synchronize()
+        res = np.concatenate([m.moments().ravel() for m in mem])
+        b.close()
+        return res
+    out["batch_q27_8rows"] = lambda: batch27(8)
+    out["batch_q27_14rows"] = lambda: batch27(14)
+
     def batch():
         b = mrlbm.Batch(mrlbm.D3Q19, mrlbm.F16)
         mem = []
