@@ -425,16 +425,23 @@ static bool dense_domain(const mrlbm_domain* dom)
 }
 
 // Whether the D3Q27 bulk sets run in the sums march: always with FP32 moments.
-// 16-bit ones cost it a conversion of each of the rows it reads, so it gains
-// only where many tiles hide its longer steps (256^3 FP16 2,501 us per 10
-// steps against 2,827; 100 x 90 x 80, 20 steps, 456 against 442 at the same
-// chunk, 743 against 549 alone).  The line is drawn at the cross-section, 256
-// columns, so that the slabs of a domain cut in z run the kernel of the whole.
+// 16-bit ones cost it a conversion of each of the rows it reads, which pays
+// only where many tiles hide its longer steps: where the columns alone, in one
+// chunk, make 1.4 waves of its CTAs.  Measured (us a step of the populations
+// against the sums, FP16, alone / among others): 384 x 384 x 16, 576 columns,
+// 48.7 / 47.8 against 52.2 / 49.3; 256 x 256 x 8, 256 columns, 17.0 / 13.6
+// against 23.4 / 14.8; 512 x 384 (768 columns) 38.9 / 39.3 against 36.9 / 36.8
+// at 8 planes, 217 / 208 against 184 / 180 at 64; split FP16 there 45.6 / 45.1
+// against 44.3 / 43.7 at 8, 72.5 / 70.6 against 71.9 / 69.8 at 16.  (Below the
+// line the sums win too on deep domains, 256 x 256 x 200 FP16 313 / 222
+// against 202 / 199, and lose on shallow ones; but the line is drawn at the
+// cross-section, so that the slabs of a domain cut in z run the kernel of the
+// whole.)
 static bool sums_domain(const mrlbm_domain* dom)
 {
     const mrlbm_desc& d = dom->d;
-    return d.storage == MRLBM_F32 ||
-           (long long)((d.nx + TILE_X - 1) / TILE_X) * ((d.ny + TYI_BULK - 1) / TYI_BULK) >= 256;
+    const long long cols = (long long)((d.nx + TILE_X - 1) / TILE_X) * ((d.ny + TYI_BULK - 1) / TYI_BULK);
+    return d.storage == MRLBM_F32 || 5 * cols >= 7LL * dom->nsm * SUM_CTAS;
 }
 
 // z planes per CTA of the sums march: even chunks of at most 32 planes (48 with

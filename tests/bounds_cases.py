@@ -43,7 +43,9 @@ def cases():
     out = {}
     for shape, q, st in [((33, 9, 5), 27, mrlbm.F32), ((32, 8, 3), 27, mrlbm.F32), ((1, 12, 10), 19, mrlbm.F32),
                          ((65, 17, 2), 27, mrlbm.F32), ((2, 2, 2), 27, mrlbm.F32), ((31, 7, 4), 19, mrlbm.F16),
-                         ((40, 10, 6), 27, mrlbm.F16U)]:
+                         ((40, 10, 6), 27, mrlbm.F16U),
+                         # over the 1.4 waves of columns from which 16-bit D3Q27 boxes take the sums march
+                         ((512, 312, 2), 27, mrlbm.F16), ((514, 313, 1), 27, mrlbm.F16U)]:
         nx, ny, nz = shape
         out["bulk_%dx%dx%d_q%d_s%d" % (nx, ny, nz, q, st)] = lambda nx=nx, ny=ny, nz=nz, q=q, st=st: _run(
             mrlbm.make_desc(nx, ny, nz, lattice=q, storage=st, tau=0.7))

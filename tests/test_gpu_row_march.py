@@ -59,13 +59,56 @@ def test_d3q27_bulk(shape, force):
 @pytest.mark.parametrize("storage,ulp", [(mrlbm.F16, 2.0 ** -11), (mrlbm.BF16, 2.0 ** -8), (mrlbm.F16U, 2.0 ** -20)])
 @pytest.mark.parametrize("shape", [(33, 9, 2), (512, 120, 2), (512, 128, 2), (515, 130, 3)])
 def test_d3q27_16bit(shape, storage, ulp):
-    """Both sides of the cross-section from which 16-bit moments take the sums
-    march (256 columns of 32 x 8 nodes)."""
+    """16-bit boxes of few and of 256 columns of 32 x 8 nodes (the line from
+    which they take the sums march: test_16bit_one_step)."""
     d = mrlbm.make_desc(*shape, lattice=mrlbm.D3Q27, storage=storage, tau=0.6)
     low, second = errors(d)
     # split storage keeps the second moments (and the little they give u) in one fp16 word
     assert low < STEPS * max(ulp, 2.0 ** -14 if storage == mrlbm.F16U else 0.0), low
     assert second < 4 * STEPS * max(ulp, 2.0 ** -11), second
+
+
+# unit roundoff of a stored word; velocity of the split storage: two words
+UNIT = {mrlbm.F32: 2.0 ** -24, mrlbm.F16: 2.0 ** -11, mrlbm.BF16: 2.0 ** -8, mrlbm.F16U: 2.0 ** -11}
+
+
+def one_step(d, seed, dev):
+    """|error| after one step over its bound, the largest of each moment: the
+    start is read back as stored, so a moment is off by the rounding of its
+    own new word, unit * |moment|, and by FP32 sums of whole populations, 64 eps
+    (times the stored scaling 3, 4.5 or 9).  Density deviations of `dev` are
+    well over both."""
+    shape = (d.nz, d.ny, d.nx)
+    rng = np.random.default_rng(seed)
+    dom = mrlbm.Domain(d)
+    dom.init_flow(1 + dev * rng.standard_normal(shape), *(0.02 * rng.standard_normal((3,) + shape)))
+    orc = pu.oracle_for(d)
+    orc.set_moments(pu.gpu_to_oracle_layout(dom.moments()))
+    dom.step(1)
+    orc.step(1)
+    got, want = pu.gpu_to_oracle_layout(dom.moments()), np.asarray(orc.moments(), dtype=np.float64)
+    dom.close()
+    out = []
+    for k in range(10):
+        unit = 2.0 ** -22 if d.storage == mrlbm.F16U and 1 <= k <= 3 else UNIT[d.storage]
+        scale = 1.0 if k == 0 else 3.0 if k <= 3 else 9.0
+        # 64 eps: the sums; the smallest words of FP16 (2^-24 over the storage scale of 8 at least)
+        bound = unit * np.abs(want[..., k]) * (1 + 1e-3) + 64 * EPS * scale
+        out.append(float(np.max(np.abs(got[..., k] - want[..., k]) / bound)))
+    assert np.sqrt(np.mean(want[..., 0] ** 2)) > 0.5 * dev   # the deviations are there to be seen
+    return out
+
+
+@pytest.mark.parametrize("force", [False, True])
+@pytest.mark.parametrize("storage", [mrlbm.F16, mrlbm.BF16, mrlbm.F16U])
+@pytest.mark.parametrize("shape", [(33, 9, 2), (512, 304, 2), (512, 312, 2), (520, 330, 3)])
+def test_16bit_one_step(shape, storage, force):
+    """608, 624 and 714 columns of 32 x 8 nodes: both sides of the 1.4 waves of
+    CTAs from which 16-bit moments take the sums march."""
+    f = (2e-4, -1e-4, 3e-4) if force else (0.0, 0.0, 0.0)
+    d = mrlbm.make_desc(*shape, lattice=mrlbm.D3Q27, storage=storage, tau=0.6, force=f)
+    over = one_step(d, 3, 0.02)
+    assert max(over) < 1.0, over
 
 
 @pytest.mark.parametrize("nz", [2660, 2700])   # 4 columns: under and over 24 planes a CTA's place (10,656)
