@@ -444,35 +444,41 @@ static bool sums_domain(const mrlbm_domain* dom)
     return d.storage == MRLBM_F32 || 5 * cols >= 7LL * dom->nsm * SUM_CTAS;
 }
 
-// z planes per CTA of the sums march: even chunks of at most 32 planes (48 with
+// z planes per CTA of the sums march: chunks of at most 32 planes (48 with
 // 16-bit moments: 256^3 FP16 32 / 43 / 64 planes 262 / 250 / 248 us a step)
-// that make 1.4 waves of CTAs; a domain that has not as many at 11 planes takes the
-// shortest chunk up to there that fits one wave.  Longer chunks save their two lead planes
+// that make 1.4 waves of CTAs, but not under 11 planes for that; a domain that
+// has not as many at 11 takes the shortest chunk up to there that fits one
+// wave (11 itself where none does).  The planes are then spread evenly over
+// that many chunks.  Longer chunks save their two lead planes
 // (6 % at 32), but neighbouring columns then drift apart and re-read their
 // halo rows from DRAM instead of L2, and a step of few tiles waits for whole
 // columns.  Measured (us a step, alone): 256^3 FP32 24 / 32 / 43 / 64 / 128
 // planes 279 / 274 / 283 / 327 / 379; 512^3 FP16 64 / 256 planes 1,745 /
 // 2,519; 128^3 FP32 13 / 16 / 20 / 32 planes 41.5 / 45.2 / 47.4 / 61.7; 64^3
 // 3 / 4 / 8 planes 11.7 / 13.6 / 18.9 (among others 7.6 / 6.7 / 7.1; the 27
-// populations at 4 planes 12.5 and 8.9); 99 x 62 x 139, 60 steps, 8 / 10 / 11 /
-// 14 planes 1,578 / 1,570 / 1,541 / 1,808 (among others 1,464 / 1,358 / 1,320 /
-// 1,238); 128 x 100 x 90, 40 steps, 8 / 11 / 14 planes 1,184 / 1,225 / 1,337
-// (among others 1,083 / 1,012 / 979).
+// populations at 4 planes 12.5 and 8.9); 32^3 1 / 2 planes 6.8 / 8.0 (among
+// others 2.9 / 3.2; the populations 6.9 and 3.2).  The 11 was tuned on boxes of
+// 48 and 52 columns, and trades one against the other there: 99 x 62 x 139, 60
+// steps, 8 / 10 / 11 / 14 planes 1,578 / 1,570 / 1,541 / 1,808 (among others
+// 1,464 / 1,358 / 1,320 / 1,238); 128 x 100 x 90, 40 steps, 8 / 11 / 14 planes
+// 1,184 / 1,225 / 1,337 (among others 1,083 / 1,012 / 979).
 int mrlbm::choose_lz_sums(const mrlbm_domain* dom)
 {
     const mrlbm_desc& d = dom->d;
     const long long cols = (long long)((d.nx + TILE_X - 1) / TILE_X) * ((d.ny + TYI_BULK - 1) / TYI_BULK);
     const long long slots = (long long)dom->nsm * SUM_CTAS;
-    auto ctas = [&](int lz) { return cols * ((d.nz + lz - 1) / lz); };
-    const int most = d.storage == MRLBM_F32 ? 32 : 48, nzc = (d.nz + most - 1) / most;
-    int lz = (d.nz + nzc - 1) / nzc;
+    auto even = [&](int n) { return (d.nz + n - 1) / n; };   // planes of each of n chunks
+    auto chunks = [&](int lz) { return (d.nz + lz - 1) / lz; };
+    auto ctas = [&](int lz) { return cols * chunks(lz); };
+    const int most = d.storage == MRLBM_F32 ? 32 : 48;
+    int lz = even(chunks(most));
     while (lz > 11 && 5 * ctas(lz) < 7 * slots) lz--;
-    if (5 * ctas(lz) < 7 * slots && lz <= 11) {
+    if (5 * ctas(lz) < 7 * slots) {   // lz is 11 at most
         const int top = lz;
-        lz = std::min(2, top);
+        lz = 1;
         while (lz < top && ctas(lz) > slots) lz++;
     }
-    return lz;
+    return even(chunks(lz));
 }
 
 bool mrlbm::tile_ordered(const mrlbm_domain* dom, int flags)

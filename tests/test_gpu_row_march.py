@@ -186,3 +186,15 @@ def test_scattered_obstacles(lattice, rheology, fill):
                         nnf_n=0.9)
     low, second = wall_errors(d, nt)
     assert low < 2 * WALL_LOW and second < 2 * WALL_SECOND, (low, second)
+
+
+@pytest.mark.parametrize("shape,planes", [((32, 32, 32), 1), ((512, 8, 8), 1), ((40, 40, 40), 1), ((48, 48, 48), 2),
+                                          ((128, 128, 128), 13), ((99, 62, 139), 11), ((256, 256, 256), 32),
+                                          ((160, 160, 160), 23)])
+def test_sums_march_chunks(shape, planes):
+    """Few tiles: the shortest chunk of one wave, one plane if that fits; the
+    planes evenly spread over the chunks (128: ten of 13, not nine of 14 and
+    one of 2)."""
+    dom = mrlbm.Domain(mrlbm.make_desc(*shape, lattice=mrlbm.D3Q27, tau=0.6))
+    assert dom.z_chunk() == planes
+    dom.close()
