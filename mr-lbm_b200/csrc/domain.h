@@ -89,6 +89,7 @@ inline bool is_half_storage(int storage) { return storage == MRLBM_F16 || storag
 mrlbm_status domain_alloc(mrlbm_domain* dom);
 int choose_lz(const mrlbm_domain* dom, int tyi, int ctas);
 int choose_lz_overlap(const mrlbm_domain* dom, int tyi, int ctas);
+int choose_lz_dense(const mrlbm_domain* dom);
 int choose_lz_sums(const mrlbm_domain* dom);
 // whether a step with these flags is tile-ordered (overlapping launches)
 bool tile_ordered(const mrlbm_domain* dom, int flags);

@@ -367,7 +367,7 @@ mrlbm_status mrlbm::domain_alloc(mrlbm_domain* dom)
     dom->dense = dense_domain(dom);
     dom->sums = sums_domain(dom);
     dom->lz_b[0] = choose_lz(dom, TYI_BULK, step_ctas(19, F_DENSE, TYI_BULK));
-    dom->lz_b[1] = choose_lz_overlap(dom, TYI_BULK, step_ctas(19, F_DENSE, TYI_BULK));
+    dom->lz_b[1] = choose_lz_dense(dom);
     return MRLBM_OK;
 }
 
@@ -442,6 +442,38 @@ static bool sums_domain(const mrlbm_domain* dom)
     const mrlbm_desc& d = dom->d;
     const long long cols = (long long)((d.nx + TILE_X - 1) / TILE_X) * ((d.ny + TYI_BULK - 1) / TYI_BULK);
     return d.storage == MRLBM_F32 || 5 * cols >= 7LL * dom->nsm * SUM_CTAS;
+}
+
+// z planes per CTA of tile-ordered F_DENSE steps: the even chunks of at most 32
+// planes (48 with 16-bit moments) that minimise the chunk's time, its planes
+// and two lead planes and a start-up of about 5, times the waves of CTAs and
+// half of one for the last (fitted on 27 boxes of 144^3 to 340^3: within 4 % of
+// the best even chunk, 0.8 % on average).  Chunks as long as one wave or
+// choose_lz_overlap asks for let neighbouring columns drift apart, and leave a
+// step's few long CTAs for the next one to wait on.  us a step alone (among
+// others), two CTAs an SM / three with those chunks / with these: FP32 160^3
+// 32 / 40 / 20 planes 70.7 (67.6) / 87.9 (63.9) / 66.0 (65.5); 224^3 75 / 112 /
+// 32 planes 195 (172) / 247 (214) / 167 (165); 340^3 85 / 85 / 31 planes 623
+// (614) / 715 (724) / 584 (583); FP16 96 x 300 x 120 24 / 40 / 20 planes 63.3
+// (63.1) / 79.9 (54.6) / 59.4 (57.9).
+int mrlbm::choose_lz_dense(const mrlbm_domain* dom)
+{
+    const mrlbm_desc& d = dom->d;
+    const long long cols = (long long)((d.nx + TILE_X - 1) / TILE_X) * ((d.ny + TYI_BULK - 1) / TYI_BULK);
+    const long long slots = (long long)dom->nsm * step_ctas(19, F_DENSE, TYI_BULK);
+    const int most = d.storage == MRLBM_F32 ? 32 : 48;
+    int best = 1;
+    long long best_cost = -1;
+    for (int n = (d.nz + most - 1) / most; n <= d.nz; n++) {
+        const int lz = (d.nz + n - 1) / n;
+        const long long ctas = cols * ((d.nz + lz - 1) / lz);
+        const long long cost = (lz + 2 + 5) * (2 * ctas + slots);
+        if (best_cost < 0 || cost < best_cost) {
+            best_cost = cost;
+            best = lz;
+        }
+    }
+    return best;
 }
 
 // z planes per CTA of the sums march: chunks of at most 32 planes (48 with

@@ -111,6 +111,26 @@ def test_16bit_one_step(shape, storage, force):
     assert max(over) < 1.0, over
 
 
+@pytest.mark.parametrize("force", [False, True])
+@pytest.mark.parametrize("storage", [mrlbm.F32, mrlbm.F16, mrlbm.BF16])
+@pytest.mark.parametrize("nz", [2660, 2700])   # as in test_d3q19_dense
+def test_d3q19_dense_one_step(nz, storage, force):
+    f = (2e-4, -1e-4, 3e-4) if force else (0.0, 0.0, 0.0)
+    d = mrlbm.make_desc(33, 9, nz, lattice=mrlbm.D3Q19, storage=storage, tau=0.6, force=f)
+    over = one_step(d, 4, 0.02)
+    assert max(over) < 1.0, over
+
+
+@pytest.mark.parametrize("shape,planes", [((160, 160, 160), 20), ((96, 300, 120), 20), ((224, 224, 224), 32),
+                                          ((203, 173, 121), 25), ((340, 340, 24), 24)])
+def test_d3q19_dense_chunks(shape, planes):
+    """Not the one wave of long chunks, nor a few waves of them (40, 40, 112
+    planes here once)."""
+    dom = mrlbm.Domain(mrlbm.make_desc(*shape, lattice=mrlbm.D3Q19, tau=0.6))
+    assert dom.z_chunk() == planes
+    dom.close()
+
+
 @pytest.mark.parametrize("nz", [2660, 2700])   # 4 columns: under and over 24 planes a CTA's place (10,656)
 def test_d3q19_dense(nz):
     """The three-CTA shape of the D3Q19 bulk step, against the oracle, and bit
