@@ -322,12 +322,14 @@ mrlbm_status mrlbm_save_macr_bin(mrlbm_domain* dom, const char* path_files, cons
  * (src/saveData.cu:303-400): rho, velocity (physical u), omega when present;
  * <path>/<id>/<id>_vtk<step>.vtk (src/saveData.cu:153). */
 mrlbm_status mrlbm_save_vtk(mrlbm_domain* dom, const char* path_files, const char* id_sim, int step);
-/* <path>/<id>/<id>_info.txt (src/saveData.cu:469-613); case_name = BC type. */
+/* <path>/<id>/<id>_info.txt (src/saveData.cu:469-613); case_name = BC type.
+ * BY and BZ are the rows and z planes of the CTAs that step the domain. */
 mrlbm_status mrlbm_save_info(mrlbm_domain* dom, const char* path_files, const char* id_sim,
                              const char* case_name, int nsteps, double mlups);
 /* The same text for a description alone, on the host (no device work; BY and
- * BZ are the step geometry of the description without wall classes on a
- * 148-SM B200): *len receives its length; buf (may be NULL to query) must hold
+ * BZ are nominal, those of the plain march of the description without wall
+ * classes on a 148-SM B200, where a domain's own file has those that it is
+ * stepped with): *len receives its length; buf (may be NULL to query) must hold
  * len + 1 bytes. */
 mrlbm_status mrlbm_info_text(const mrlbm_desc* desc, const char* id_sim, const char* case_name, int nsteps,
                              double mlups, char* buf, size_t cap, size_t* len);

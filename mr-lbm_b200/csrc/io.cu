@@ -377,16 +377,15 @@ extern "C" mrlbm_status mrlbm_save_info(mrlbm_domain* dom, const char* path_file
     StepArgs sa;
     int flags = 0;
     fill_step_args(dom, sa, dom->cur, flags);
-    // the nominal tile of the flag set (the bulk sets have z chunks of their own), as in mrlbm_info_text
-    const int kind = tile_kind(tile_rows(flags));
-    const int lz = dom->lz > 0 ? dom->lz : tile_ordered(dom, flags) ? dom->lz_o[kind] : dom->lz_t[kind];
-    const std::string t = info_text(dom->d, id_sim, case_name, nsteps, mlups, tile_rows(flags), lz);
+    const std::string t = info_text(dom->d, id_sim, case_name, nsteps, mlups, tile_rows(flags), sa.lz);
     return write_file(std::string(path_files) + "/" + id_sim + "/" + id_sim + "_info.txt", t.data(), t.size());
 }
 
-// The same text for a description alone, on the host (no device work): the
-// step's geometry is that of a domain without wall classes on a 148-SM B200,
-// stepped tile-ordered (the default).
+// The same text for a description alone, on the host (no device work).  BY and
+// BZ are nominal: those of the two-CTA population march on a 148-SM B200 for a
+// domain without wall classes, stepped tile-ordered (the default).  The sums
+// march and the three-CTA shape have z chunks of their own, which the file of a
+// domain (mrlbm_save_info) reports.
 extern "C" mrlbm_status mrlbm_info_text(const mrlbm_desc* d, const char* id_sim, const char* case_name, int nsteps,
                                         double mlups, char* buf, size_t cap, size_t* len)
 {
