@@ -76,7 +76,7 @@ mrlbm_status build_bc_class(int q, int mq, uint32_t word, const double uvel[4][3
 // geom: the domain's shape and the populations of its resting ghost shell, for
 // the classes that take the total sums (BC_TOTALS); null: none does
 struct WallGeom {
-    int nx, ny, nz;
+    int nx, ny;
     bool wall_x, wall_y;   // not periodic
     double fext[27];
 };

@@ -100,10 +100,6 @@ __host__ __device__ constexpr int ctas_per_sm(int tyi) { return tyi <= 8 ? 2 : 1
 // CTA per SM, else an even share of the SM's 228 KB less the 1 KB each
 // block reserves
 __host__ __device__ constexpr size_t smem_share(int ctas) { return ctas == 1 ? 232448 : 233472 / ctas / 128 * 128 - 1024; }
-__host__ __device__ constexpr size_t smem_budget(int tyi)
-{
-    return smem_share(ctas_per_sm(tyi));
-}
 // stored moments and moment pairs of a flag set
 __host__ __device__ constexpr int nmoments_of(int flags)
 {
@@ -190,6 +186,7 @@ struct alignas(16) BcClass {
     uint32_t pad[4];
 };
 static_assert(sizeof(BcClass) == 336, "BcClass is read as float4 words");
+constexpr int STAGED_MIN = 37;   // classes that every kernel with a staged table holds (the fewest: FP32 batches at 8 rows)
 
 struct StepArgs {
     void* __restrict__ m_out;         // padded planes [nm][nz+2][ny+2][pitch]
@@ -1440,6 +1437,7 @@ struct ZSmem {
         return n;
     }
     static constexpr int CT = ct_fit();
+    static_assert(!WC || CT >= STAGED_MIN, "classify_nodes leaves a table of STAGED_MIN classes unsorted");
     static constexpr size_t ct_bytes = ct_bytes_of(CT);
     static constexpr size_t bytes = ring_bytes + ct_bytes;
     static_assert(bytes <= budget, "shared memory over the sm_100 limit");
@@ -1940,9 +1938,10 @@ __host__ __device__ constexpr int step_warps(int q, int flags, int tyi)
 }
 // F_DENSE: the D3Q19 bulk sets (five pairs) fit three CTAs an SM with 64
 // registers a thread and a ring of three stages; two CTAs keep 72 and four.
-// Measured (us, among others / alone): ragged 203 x 173 x 121 box, 20 steps,
-// 1,543 / 1,676 against 1,624 / 1,706; 256^3, 10 steps, 2,730 / 2,891 against
-// 2,851 / 2,916.  A domain of few tiles runs alone slower with them (64^3, 50
+// Measured (us a step, alone / among others, three CTAs against two): ragged
+// 203 x 173 x 121 box 70.9 / 68.6 against 75.9 / 75.4; 256^3 246 / 244 against
+// 256 / 253; 144^3 FP16, near the line of dense_domain, 52.4 / 52.2 against
+// 71.2 / 52.0.  A domain of few tiles runs alone slower with them (64^3, 50
 // steps, 664 against 561; 128^3 FP16, 20 steps, 789 against 787 at its best
 // chunk), so small ones keep two: dense_domain.
 __host__ __device__ constexpr int step_ctas(int q, int flags, int tyi)

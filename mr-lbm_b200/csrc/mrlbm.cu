@@ -644,7 +644,7 @@ static double stored_value(const mrlbm_domain* dom, int m)
 static WallGeom wall_geom(const mrlbm_domain* dom)
 {
     const mrlbm_desc& d = dom->d;
-    WallGeom g{d.nx, d.ny, d.nz, !d.periodic[0], !d.periodic[1], {}};
+    WallGeom g{d.nx, d.ny, !d.periodic[0], !d.periodic[1], {}};
     double m[10];
     for (int k = 0; k < 10; k++) m[k] = stored_value(dom, k);
     for (int i = 0; i < dom->q; i++) {
@@ -725,9 +725,9 @@ mrlbm_status mrlbm::classify_nodes(int q, int mq, const uint32_t* nt, long long 
     }
     // The wall kernels stage the first classes of the table in shared memory:
     // put those of the most nodes first (a duct of scattered obstacles has all
-    // 254 masks, of which a few dozen cover most nodes).  Every kernel holds 37
-    // classes at least, so a smaller table needs no order.
-    if (table.size() > 37) {
+    // 254 masks, of which a few dozen cover most nodes).  A table that every
+    // kernel holds whole needs no order.
+    if (table.size() > STAGED_MIN) {
         long long count[256] = {};
         for (long long k = 0; k < n; k++) count[cls[k]]++;
         std::vector<int> order(table.size() - 1);

@@ -1,5 +1,5 @@
 // step_dispatch.cuh -- launch of the z-marching step kernel for one
-// (lattice, storage) pair; instantiated in step_q*_*.cu so the 36 kernel
+// (lattice, storage) pair; instantiated in step_q*_*.cu so the kernel
 // variants compile in parallel translation units.
 #pragma once
 #include <cuda_runtime.h>

@@ -338,9 +338,13 @@ __device__ __forceinline__ F2 p_inv(F2 v) { return f2_pack(1.0f / row_of(v, 0), 
 // x + 1), the node's own c_x = 0 lines U0; o: the stored moments 0 .. 9.
 // The sums carry 6^3 = 216 times the moments.  Stored scaling: 3u = 3 j / rho,
 // 9 Pi_ij = 9 P_ij / rho, 4.5 Pi_ii = (4.5 P_ii - 1.5 (rho - rho0)) / rho with
-// P_ii the deviation from rho0 / 3; all from the one quotient 1 / (72 rho)
-// by exact factors (a rounded 1 / 216 would scale the velocity by the same
-// 1 + 1e-8 every step).  The collision is collide_scaled's.
+// P_ii the deviation from rho0 / 3; all from the quotient 1 / (72 rho) and its
+// rounded multiples by 3 and 72, so a velocity meets the roundings of one
+// quotient, which vary with the density, and the density deviation that of
+// 1 / 216.  Drift of the sums over 20,000 steps of 32^3 boxes, here / with the
+// 27 populations: mean density deviation 1.2e-5 / 1.6e-3 of itself (noise),
+// 1.2e-4 / 1.1e-2 (waves), momentum 2.5e-5 / 1.4e-5 (shear), 4e-6 / 4.8e-5.
+// The collision is collide_scaled's.
 template <int FLAGS, typename P>
 __device__ __forceinline__ void x_collide(const StepArgs& a, const P (&fl)[6], const P (&fr)[6], const P (&U0)[6],
                                           P (&o)[10])
