@@ -63,6 +63,26 @@ def test_lid_cavity_d3q19_walls_on_every_face():
     assert np.array_equal(got, want)
 
 
+@pytest.mark.parametrize("storage", [mrlbm.F32, mrlbm.F16])
+def test_lid_cavity_d3q27_walls_on_every_face(storage):
+    """Classes that take the total sums (x and y faces) next to a slab's ghost
+    planes, whose own x and y shells they read."""
+    d = mrlbm.lid_cavity_desc(40, re=50.0, lid_u=0.05, lattice=mrlbm.D3Q27, storage=storage, ny=18, nz=23)
+    nt = mrlbm.lid_cavity_node_types(40, 18, 23, 1)
+    want, got, _ = _run_both(d, 3, 30, nt=nt)
+    assert np.array_equal(got, want)
+
+
+@pytest.mark.parametrize("shape,lattice,storage", [((512, 304, 6), 27, mrlbm.F16), ((512, 312, 6), 27, mrlbm.F16),
+                                                   ((512, 312, 6), 27, mrlbm.F16U), ((33, 9, 2700), 19, mrlbm.F32)])
+def test_slabs_of_a_box_at_the_line_of_a_kernel(shape, lattice, storage):
+    """16-bit D3Q27 boxes under and over the columns from which they run in
+    sums, and a D3Q19 box that takes three CTAs an SM where its slabs take two."""
+    d = mrlbm.make_desc(*shape, lattice=lattice, storage=storage, tau=0.6)
+    want, got, _ = _run_both(d, 2, 6)
+    assert np.array_equal(got, want)
+
+
 def test_half_storage_vortex():
     d = mrlbm.make_desc(48, 40, 36, lattice=mrlbm.D3Q19, storage=mrlbm.F16, tau=0.55)
     want, got, _ = _run_both(d, 2, 20, init=lambda dom: dom.init_taylor_green(0.04, 36 / (2 * np.pi)))
